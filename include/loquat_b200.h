@@ -256,12 +256,12 @@ int lq_sim_renewal_launches(void* sim, int* launches);
  * 4 = 128 x 7.  7-10: one thread per target in tile order (the targets of a
  * block form a compact box of cells, so its neighbours stay in L1; the
  * order is rebuilt after every search): 7 = 768 x 1, 8 = 384 x 2,
- * 9 = 640 x 1, 10 = 320 x 2.  All of these give bit-identical results.
+ * 9 = 256 x 3, 10 = 320 x 2.  All of these give bit-identical results.
  * 5, 6: warp-cooperative, 8 or 32 lanes share a target's list and combine
  * their sums with shuffle reductions (for small cases); the summation
  * order differs, so results agree to rounding.  A new simulation starts
- * with shape 9 when its material particles fill four waves of 640-thread
- * blocks on every SM, else with shape 0.  No reference counterpart. */
+ * with shape 9 from 2560 material particles per SM on, else with
+ * shape 0.  No reference counterpart. */
 int lq_sim_set_pair_shape(void* sim, int shape);
 int lq_sim_pair_shape(void* sim, int* shape);
 /* Autotuner: times `steps` steps for each pair kernel shape at the current

@@ -74,8 +74,8 @@ template <bool kPk>
 __device__ __forceinline__ void pack_slot(const NbrArrays& nb, int i, const float4& x, const float4& v,
                                           const tensor2d& s)
 {
-    if (!nb.xr) return;
-    nb.xr[i] = make_float4(x.x, x.y, x.z, v.w);
+    if (!nb.xs) return;
+    nb.xs[2 * (size_t)i] = make_float4(x.x, x.y, x.z, v.w);
     store_packed<kPk>(nb, i, v, s);
 }
 
@@ -406,7 +406,7 @@ int launch_predict(const Parameters* ph, const Parameters* pd, const State& in, 
      * more registers than the other models' kernels */
     const bool vwm = ph->constitutive_model == 3;
     const int nb = blocks_for(ph->np, kBlock);
-    const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr, nullptr};
+    const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     if (in.xlo && out.xlo) {
         if (vwm) k_predict<true, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, vw, pk,
                                                               stage);
@@ -431,7 +431,7 @@ int launch_correct(const Parameters* ph, const Parameters* pd, const State& cur,
     k_correct<false, false><<<blocks_for(ph->npm, kBlock), kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, ini_idx, cur, r, health,
                                                              VerletCheck{nullptr, nullptr, 0.0f, 0.0f, nullptr, 0.0f}, ph->npb,
                                                              MaterialTable(), MaterialTable(),
-                                                             NbrArrays{nullptr, nullptr, nullptr, nullptr});
+                                                             NbrArrays{nullptr, nullptr, nullptr});
     LQ_TRY_CUDA(cudaGetLastError(), "k_correct");
     return LQ_OK;
 }
@@ -452,7 +452,7 @@ int launch_correct_into(const Parameters* ph, const Parameters* pd, const State&
     /* material slots only: boundary slots are written by Adami into both
      * buffers */
     const int nb = blocks_for(ph->npm, kBlock), f = ph->npb;
-    const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr, nullptr};
+    const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     if (cur.xlo && ini.xlo && out.xlo) {
         if (vwm) k_correct<true, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);
         else k_correct<true, false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);

@@ -538,23 +538,33 @@ __device__ __forceinline__ int vw_update_d(const VWConst& c, double dt, const te
 
 /* Packed neighbour data for the list pair kernel: dense arrays over all
  * slots, with s = sigma / rho^2,
- *   nb.xr[j] = (x, y, z, rho), nb.sa[j] = (sxx, syy, szz, sxy),
+ *   nb.xs[2 j] = (x, y, z, rho), nb.xs[2 j + 1] = (sxx, syy, szz, sxy),
  *   nb.sb[j] = (sxz, syz, v0, v1),
  * where the plain form keeps (v0, v1) = (vx, vy) and vz in nb.vz[j]
- * (52 bytes per particle, four gathers per pair) and the mixed form packs
- * the whole velocity into v0, v1 (pack_velocity: 48 bytes, three 16-byte
- * gathers per pair).  The pair kernel is bound by the L1 data pipe: a
- * warp's gathered neighbours sit close together in memory and the pipe's
- * work follows the load instructions and the sectors each gathers, so the
- * record holds only the 13 values a pair needs (no pressure word of
- * pospres, no 24-byte stress records read as three 8-byte loads).
- * 1 / rho is formed as the state-array pair body forms it. */
+ * (52 bytes per particle, three gathers per pair) and the mixed form packs
+ * the whole velocity into v0, v1 (pack_velocity: 48 bytes, two gathers per
+ * pair).  The pair kernel's time follows the number of gathers and their
+ * passes over the L1 banks more than the bytes: the first two words come
+ * with one 32-byte load, which is one full sector, instead of one load
+ * each.  On the 1.97 M-particle cylinder (mixed form, lists in bank order)
+ * the launch takes 602 us so and 640 with three 16-byte gathers (24 warps
+ * per SM); a fourth gather of 4 bytes in place of the packed velocity's ten
+ * instructions costs 70 us.  1 / rho is formed as the state-array pair body
+ * forms it.
+ */
 struct NbrArrays {
-    float4* xr;
-    float4* sa;
+    float4* xs;
     float4* sb;
     float* vz;
 };
+
+/* Slot j's (x, y, z, rho) and (sxx, syy, szz, sxy) in one 32-byte load. */
+__device__ __forceinline__ void load_xs(const NbrArrays& nb, int j, float4& xr, float4& sa)
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(xr.x), "=f"(xr.y), "=f"(xr.z), "=f"(xr.w), "=f"(sa.x), "=f"(sa.y), "=f"(sa.z), "=f"(sa.w)
+        : "l"(nb.xs + 2 * (size_t)(unsigned)j));
+}
 
 /* The mixed form's gathered velocity in two words (lq_pack.h: a shared
  * exponent and three 18-bit mantissas). */
@@ -580,7 +590,7 @@ __device__ __forceinline__ void store_packed(const NbrArrays& nb, int i, const f
 {
     const float rinv = __fdividef(1.0f, v.w);
     const float r2 = rinv * rinv;
-    nb.sa[i] = make_float4(str.xx * r2, str.yy * r2, str.zz * r2, str.xy * r2);
+    nb.xs[2 * (size_t)i + 1] = make_float4(str.xx * r2, str.yy * r2, str.zz * r2, str.xy * r2);
     if (kPk) {
         const float2 w = pack_velocity(v.x, v.y, v.z);
         nb.sb[i] = make_float4(str.xz * r2, str.yz * r2, w.x, w.y);
@@ -597,16 +607,15 @@ __device__ __forceinline__ void store_packed_stress(const NbrArrays& nb, int i, 
 {
     const float rinv = __fdividef(1.0f, rho);
     const float r2 = rinv * rinv;
-    nb.sa[i] = make_float4(str.xx * r2, str.yy * r2, str.zz * r2, str.xy * r2);
+    nb.xs[2 * (size_t)i + 1] = make_float4(str.xx * r2, str.yy * r2, str.zz * r2, str.xy * r2);
     *reinterpret_cast<float2*>(nb.sb + i) = make_float2(str.xz * r2, str.yz * r2);
 }
 
-/* The packed arrays inside `rec` (np x 13 floats, 16-byte aligned). */
+/* The packed arrays inside `rec` (np x 13 floats, 32-byte aligned). */
 inline NbrArrays nbr_arrays(float* rec, int np)
 {
     const size_t n = (size_t)np;
-    return NbrArrays{reinterpret_cast<float4*>(rec), reinterpret_cast<float4*>(rec) + n,
-                     reinterpret_cast<float4*>(rec) + 2 * n, rec + 12 * n};
+    return NbrArrays{reinterpret_cast<float4*>(rec), reinterpret_cast<float4*>(rec) + 2 * n, rec + 12 * n};
 }
 
 }  // namespace lqb

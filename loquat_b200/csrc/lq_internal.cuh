@@ -151,7 +151,7 @@ struct NeighborList {
 /* ------------------------------------------------------------ operators */
 int launch_neighbor_list(const Parameters* par_host, const Parameters* par_dev, const float4* pos, const Cells& c,
                          const NeighborList& nl, cudaStream_t s);
-/* `rec` (np x 13 floats, 16-byte aligned; required) holds the neighbour
+/* `rec` (np x 13 floats, 32-byte aligned; required) holds the neighbour
  * data packed into dense arrays (position and density, velocity and
  * sigma/rho^2: 52 bytes per particle, 48 in the compensated form, whose
  * velocity is packed into two words) that the pair kernel gathers; with
@@ -188,7 +188,7 @@ int launch_boundary_targets(int npb, const int* count, const int* count2, int* a
  * with G lanes per target.  Shapes with the tile order take their targets
  * from TileOrder::order (launch_tile_order, after each search). */
 constexpr int kPairShapeCount = 11;
-constexpr int kDefaultTiledShape = 9;   /* 640 x 1, tile order */
+constexpr int kDefaultTiledShape = 9;   /* 256 x 3, tile order */
 extern const int kPairShapes[kPairShapeCount][3];
 /* Launch shape of a new simulation with npm material particles. */
 int default_pair_shape(int npm);
@@ -277,6 +277,9 @@ int launch_neighbor_list_range(const Parameters* par_host, const Parameters* par
 int launch_list_refresh(const Parameters* par_host, int first, int n, float cut, const float4* pos,
                         const int* inner_count, const NeighborList& shell, const NeighborList& nl, int* health,
                         cudaStream_t s);
+/* The first n targets' lists put into an order in which the pair kernel's
+ * lanes gather from different banks. */
+int launch_list_arrange(int n, const NeighborList& nl, cudaStream_t s);
 /* Fills n ints with v; adds v to one int. */
 int fill_int(int* p, int n, int v, cudaStream_t s);
 int add_int(int* p, int v, cudaStream_t s);

@@ -88,7 +88,11 @@ LQ_PACK_HD void unpack_velocity_words(unsigned w0, unsigned w1, float& vx, float
 {
     const float q = pack_float(w1 & 0x7F800000u);
     const float c = -8519680.0f * q;                       /* -(2^23 + 2^17) q */
+#if defined(__CUDA_ARCH__)
+    const unsigned uz = __funnelshift_r(w0, w1, 18) & 0x3FFFFu;
+#else
     const unsigned uz = ((w0 >> 18) | (w1 << 14)) & 0x3FFFFu;
+#endif
     vx = fmaf(pack_float((w0 & 0x3FFFFu) | 0x4B000000u), q, c);
     vy = fmaf(pack_float(((w1 >> 4) & 0x3FFFFu) | 0x4B000000u), q, c);
     vz = fmaf(pack_float(uz | 0x4B000000u), q, c);

@@ -351,6 +351,7 @@ int build_lists(LqSim* S, cudaStream_t s)
         const float cut = 2.0f * ph->h + S->skin;
         LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, S->npb, S->npm, 0, cut, S->S.pos, cells, S->nlm, S->health,
                                                s, S->S.idep, S->fr));
+        LQ_TRY(lqb::launch_list_arrange(S->npm, S->nlm, s));
         LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, 0, S->npb, 1, cut, S->S.pos, cells, S->nlb, S->health, s,
                                                S->S.idep, S->fr));
         return lqb::launch_boundary_targets(S->npb, S->nlb.count, nullptr, S->bact, S->nbact, S->bsel_tmp,
@@ -362,6 +363,7 @@ int build_lists(LqSim* S, cudaStream_t s)
     const lqb::NeighborList ib{S->nlb.list, S->inner_b, S->nlb.stride};
     LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, S->npb, S->npm, 0, cut, S->S.pos, cells, im, S->health, s,
                                            S->S.idep, S->fr, &S->wlm, inner));
+    LQ_TRY(lqb::launch_list_arrange(S->npm, im, s));   /* the inner parts: renewals append to them as they come */
     LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, 0, S->npb, 1, cut, S->S.pos, cells, ib, S->health, s, S->S.idep,
                                            S->fr, &S->wlb, inner));
     return lqb::launch_boundary_targets(S->npb, S->inner_b, S->wlb.count, S->bact, S->nbact, S->bsel_tmp,
@@ -1477,10 +1479,11 @@ extern "C" int lq_sim_rebuild_launches(void* sim, int* launches)
     if (!sim || !launches) return lqb::set_error(LQ_ERR_ARG, "lq_sim_rebuild_launches: null argument");
     LqSim* S = static_cast<LqSim*>(sim);
     /* count reset, hash, scatter, cell order (the scan is a library
-     * kernel), gather, copy, material list, boundary list (when npb > 0),
+     * kernel), gather, copy, material list and its order (when npm > 0),
+     * boundary list (when npb > 0),
      * full pack of the neighbour data, tile segments and fill (tiled
      * shapes; their scan is a library kernel) */
-    *launches = 4 + 1 + 1 + 1 + (S->npb > 0 ? 1 : 0) + 1 + (tiled(S) && S->npm > 0 ? 2 : 0);
+    *launches = 4 + 1 + 1 + (S->npm > 0 ? 2 : 0) + (S->npb > 0 ? 1 : 0) + 1 + (tiled(S) && S->npm > 0 ? 2 : 0);
     /* with two-level lists the lists the stages read are renewed from the
      * wide ones right after */
     int renewal = 0;

@@ -61,27 +61,28 @@ inline int blocks_for(long long n, int b) { return (int)((n + b - 1) / b); }
  * in the same order. */
 
 struct PairConst {
-    float ih, h, eta, m, Cg, Cw, avc, eps, wdr, cut2;
-    bool visc, artp;
+    float ih, eta, mCg, Cw, avh, eps, iwdr, cut2;
+    bool artp;
 };
 
 __device__ __forceinline__ PairConst load_pair_const(const Parameters* __restrict__ P)
 {
     PairConst K;
+    const float h = __ldg(&P->h);
     K.ih = __ldg(&P->i_h);
-    K.h = __ldg(&P->h);
     K.eta = __ldg(&P->eta);
-    K.m = __ldg(&P->m);
-    K.Cg = __ldg(&P->kernel_gradient_normalization_par);
+    /* every sum takes the factor m C' of its terms once, in rates_of */
+    K.mCg = __ldg(&P->m) * __ldg(&P->kernel_gradient_normalization_par);
     K.Cw = __ldg(&P->kernel_normalization_par);
-    K.visc = __ldg(&P->viscosity_type) == 1;
-    /* alpha * cs; zero without viscosity, so the packed pair body can
-     * evaluate the term unconditionally (it then adds exact zeros) */
-    K.avc = K.visc ? __ldg(&P->artificial_viscosity_alpha) * __ldg(&P->cs) : 0.0f;
+    /* -2 alpha cs h; zero without viscosity, so the pair body can evaluate
+     * the term unconditionally (it then adds exact zeros) */
+    K.avh = __ldg(&P->viscosity_type) == 1
+                ? -2.0f * __ldg(&P->artificial_viscosity_alpha) * __ldg(&P->cs) * h
+                : 0.0f;
     K.artp = __ldg(&P->artificial_pressure) == 1;
     K.eps = __ldg(&P->artificial_pressure_coefficient);
-    K.wdr = __ldg(&P->kernel_dr);
-    K.cut2 = 4.0f * K.h * K.h * 1.0001f; /* candidate test; the pair body applies q < 2 exactly */
+    K.iwdr = 1.0f / __ldg(&P->kernel_dr);
+    K.cut2 = 4.0f * h * h * 1.0001f; /* candidate test; the pair body applies q < 2 exactly */
     return K;
 }
 
@@ -136,124 +137,135 @@ __device__ __forceinline__ float sqrt_approx(float x)
     return r;
 }
 
-/* One pair, without branches: a pair at q >= 2 gets a zero kernel gradient
- * and adds zero to every sum.  kKahan compensates the density and
- * momentum sums. */
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+/* The factors of one pair's terms, without branches and without the common
+ * factor m C' (rates_of applies it): the density rate is t3 vr, the
+ * momentum t3 p and the velocity gradient -w (x) d.  (x_j, rho_j), v_j and
+ * s_j = sigma_j / rho_j^2 are the neighbour's.  The kernel gradient is
+ * t^3 x_ij with t = max(2 - q, 0), so a pair at q >= 2 adds zero to every
+ * sum, and a pair of a particle with itself (the filler of a list's last
+ * group) adds exact zeros: d = 0.
+ *
+ * The pair sums are bound by issue slots and the L1 data pipe, so the terms
+ * are factored to the fewest operations: t^3 multiplies v_ij . x_ij (shared
+ * by the density rate and the viscosity) and the contracted stress instead
+ * of forming the gradient's three components, the viscosity enters as a
+ * pressure on the diagonal of the stress sum, and each quotient is one
+ * reciprocal: 57 arithmetic operations a pair and three of the special
+ * function unit (about 70 and as many before; with the sums' other work
+ * 115 -> 98 instructions an entry, 758 -> 703 us a launch on the 1.97 M
+ * cylinder, 640 x 1, mixed form).  The viscosity is always evaluated (K.avh
+ * is zero without it); kArtp adds the artificial stress.  Every product and
+ * sum is contracted as written, so that all kernels that sum these terms in
+ * one order give one result. */
+struct PairFactors {
+    float t3, vr, px, py, pz, wx, wy, wz, dx, dy, dz;
+};
+
+template <bool kArtp>
+__device__ __forceinline__ PairFactors pair_factors(const PairConst& K, const Target& T, const float4& xj,
+                                                    const float3& vj, const tensor2d& sj)
+{
+    PairFactors f;
+    f.dx = T.x.x - xj.x;
+    f.dy = T.x.y - xj.y;
+    f.dz = T.x.z - xj.z;
+    const float r2 = fmaf(f.dx, f.dx, fmaf(f.dy, f.dy, f.dz * f.dz));
+    const float t = fmaxf(fmaf(-sqrt_approx(r2), K.ih, 2.0f), 0.0f);
+    f.t3 = t * t * t;
+    const float vx = T.v.x - vj.x, vy = T.v.y - vj.y, vz = T.v.z - vj.z;
+    f.vr = fmaf(vx, f.dx, fmaf(vy, f.dy, vz * f.dz));
+    /* Pi = -alpha cs h vr / ((r^2 + eta) rhobar) for vr < 0, rhobar = (rho_i + rho_j) / 2 */
+    const float pi = __fmul_rn(K.avh * fminf(f.vr, 0.0f), rcp_approx((r2 + K.eta) * (T.v.w + xj.w)));
+    float Txx = T.Sxx + sj.xx - pi, Tyy = T.Syy + sj.yy - pi, Tzz = T.Szz + sj.zz - pi;
+    const float Txy = T.Sxy + sj.xy, Txz = T.Sxz + sj.xz, Tyz = T.Syz + sj.yz;
+    if (kArtp) {
+        /* W = Cw t^4 (q + 1/2), q = 2 - t where W is not zero */
+        const float w = K.Cw * (t * f.t3) * (2.5f - t) * K.iwdr;
+        const float w4 = (w * w) * (w * w);
+        Txx = fmaf(fmaf(-K.eps, fmaxf(sj.xx, 0.0f), T.Rx), w4, Txx);
+        Tyy = fmaf(fmaf(-K.eps, fmaxf(sj.yy, 0.0f), T.Ry), w4, Tyy);
+        Tzz = fmaf(fmaf(-K.eps, fmaxf(sj.zz, 0.0f), T.Rz), w4, Tzz);
+    }
+    f.px = fmaf(Txx, f.dx, fmaf(Txy, f.dy, Txz * f.dz));
+    f.py = fmaf(Txy, f.dx, fmaf(Tyy, f.dy, Tyz * f.dz));
+    f.pz = fmaf(Txz, f.dx, fmaf(Tyz, f.dy, Tzz * f.dz));
+    const float u = f.t3 * rcp_approx(xj.w);
+    f.wx = u * vx;
+    f.wy = u * vy;
+    f.wz = u * vz;
+    return f;
+}
+
+/* A pair's density-rate and momentum terms added to (drho, ax, ay, az), its
+ * velocity-gradient terms to T. */
+__device__ __forceinline__ void add_pair(const PairFactors& f, Target& T, float& drho, float& ax, float& ay, float& az)
+{
+    drho = fmaf(f.t3, f.vr, drho);
+    ax = fmaf(f.t3, f.px, ax);
+    ay = fmaf(f.t3, f.py, ay);
+    az = fmaf(f.t3, f.pz, az);
+    T.l00 = fmaf(-f.wx, f.dx, T.l00); T.l01 = fmaf(-f.wx, f.dy, T.l01); T.l02 = fmaf(-f.wx, f.dz, T.l02);
+    T.l10 = fmaf(-f.wy, f.dx, T.l10); T.l11 = fmaf(-f.wy, f.dy, T.l11); T.l12 = fmaf(-f.wy, f.dz, T.l12);
+    T.l20 = fmaf(-f.wz, f.dx, T.l20); T.l21 = fmaf(-f.wz, f.dy, T.l21); T.l22 = fmaf(-f.wz, f.dz, T.l22);
+}
+
+/* A neighbour's packed record as it is gathered. */
+template <bool kPk>
+struct PackedRecord {
+    float4 xr, sa, sb;
+    float vz;
+};
+
+template <bool kPk>
+__device__ __forceinline__ void load_record(const NbrArrays& nb, int j, PackedRecord<kPk>& r)
+{
+    load_xs(nb, j, r.xr, r.sa);
+    r.sb = __ldg(nb.sb + j);
+    if (!kPk) r.vz = __ldg(nb.vz + j);
+}
+
+/* One pair from a gathered record. */
+template <bool kArtp, bool kPk>
+__device__ __forceinline__ void pair_terms(const PairConst& K, const PackedRecord<kPk>& r, Target& T, float& drho,
+                                           float& ax, float& ay, float& az)
+{
+    const float3 vj = kPk ? unpack_velocity(r.sb.z, r.sb.w) : make_float3(r.sb.z, r.sb.w, r.vz);
+    add_pair(pair_factors<kArtp>(K, T, r.xr, vj,
+                                 make_tensor2d(r.sa.x, r.sa.y, r.sa.z, r.sa.w, r.sb.x, r.sb.y)),
+             T, drho, ax, ay, az);
+}
+
+/* One pair from the state arrays (the walk of a target whose list
+ * overflowed), every sum compensated pair by pair with kKahan. */
 template <bool kKahan = false>
 __device__ __forceinline__ void pair_body(const PairConst& K, const State& st, Target& T, int j)
 {
-    const float4 xj = __ldg(st.pos + j);
-    const float4 vj = __ldg(st.vel + j);
-    const tensor2d sj = load_t2(st.str, j);
-    const float dx = T.x.x - xj.x, dy = T.x.y - xj.y, dz = T.x.z - xj.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float q = sqrt_approx(r2) * K.ih;
-    const float t = fmaxf(2.0f - q, 0.0f);
-    const float fac = K.Cg * t * t * t;
-    const float gx = fac * dx, gy = fac * dy, gz = fac * dz;
-    const float vx = T.v.x - vj.x, vy = T.v.y - vj.y, vz = T.v.z - vj.z;
-    if (kKahan)
-        kahan_add(T.drho, T.cdrho, vx * gx + vy * gy + vz * gz);
-    else
-        T.drho += vx * gx + vy * gy + vz * gz;
-    const float rinv = __fdividef(1.0f, vj.w);
-    const float rj2 = rinv * rinv;
-    const float Txx = T.Sxx + sj.xx * rj2, Tyy = T.Syy + sj.yy * rj2, Tzz = T.Szz + sj.zz * rj2;
-    const float Txy = T.Sxy + sj.xy * rj2, Txz = T.Sxz + sj.xz * rj2, Tyz = T.Syz + sj.yz * rj2;
-    float px = Txx * gx + Txy * gy + Txz * gz;
-    float py = Txy * gx + Tyy * gy + Tyz * gz;
-    float pz = Txz * gx + Tyz * gy + Tzz * gz;
-    if (K.visc) {
-        /* Pi = -alpha cs h vr / ((r^2 + eta) rhobar) for vr < 0 */
-        const float vr = fminf(vx * dx + vy * dy + vz * dz, 0.0f);
-        const float pi = __fdividef(-K.avc * K.h * vr, (r2 + K.eta) * (0.5f * (T.v.w + vj.w)));
-        px -= pi * gx;
-        py -= pi * gy;
-        pz -= pi * gz;
-    }
-    if (K.artp) {
-        const float wk = K.Cw * t * t * t * t * (q + 0.5f);
-        const float f = __fdividef(wk, K.wdr);
-        const float f4 = (f * f) * (f * f);
-        const float Rjx = sj.xx > 0.f ? -K.eps * sj.xx * rj2 : 0.f;
-        const float Rjy = sj.yy > 0.f ? -K.eps * sj.yy * rj2 : 0.f;
-        const float Rjz = sj.zz > 0.f ? -K.eps * sj.zz * rj2 : 0.f;
-        px += (T.Rx + Rjx) * f4 * gx;
-        py += (T.Ry + Rjy) * f4 * gy;
-        pz += (T.Rz + Rjz) * f4 * gz;
-    }
+    const float4 x = __ldg(st.pos + j);
+    const float4 v = __ldg(st.vel + j);
+    const float rinv = rcp_approx(v.w);
+    const tensor2d s = load_t2(st.str, j) * (rinv * rinv);
+    const float4 xj = make_float4(x.x, x.y, x.z, v.w);
+    const float3 vj = make_float3(v.x, v.y, v.z);
+    float d = 0.f, ax = 0.f, ay = 0.f, az = 0.f;
+    add_pair(K.artp ? pair_factors<true>(K, T, xj, vj, s) : pair_factors<false>(K, T, xj, vj, s), T, d, ax, ay, az);
     if (kKahan) {
-        kahan_add(T.ax, T.cax, px);
-        kahan_add(T.ay, T.cay, py);
-        kahan_add(T.az, T.caz, pz);
+        kahan_add(T.drho, T.cdrho, d);
+        kahan_add(T.ax, T.cax, ax);
+        kahan_add(T.ay, T.cay, ay);
+        kahan_add(T.az, T.caz, az);
     } else {
-        T.ax += px;
-        T.ay += py;
-        T.az += pz;
+        T.drho += d;
+        T.ax += ax;
+        T.ay += ay;
+        T.az += az;
     }
-    const float Vj = K.m * rinv;
-    const float wx = Vj * vx, wy = Vj * vy, wz = Vj * vz;
-    T.l00 -= wx * gx; T.l01 -= wx * gy; T.l02 -= wx * gz;
-    T.l10 -= wy * gx; T.l11 -= wy * gy; T.l12 -= wy * gz;
-    T.l20 -= wz * gx; T.l21 -= wz * gy; T.l22 -= wz * gz;
-}
-
-/* One pair from the packed arrays, its density-rate and momentum terms
- * added to (drho, ax, ay, az) and its velocity-gradient terms to T.  The
- * viscosity term is always evaluated (K.avc is zero without viscosity), so
- * a run of pairs has no branch between them; kArtp adds the artificial
- * stress.  A pair of a particle with itself (the filler of a list's last
- * group of four) adds exact zeros: r = 0 makes the kernel gradient zero. */
-template <bool kArtp, bool kPk>
-__device__ __forceinline__ void pair_terms(const PairConst& K, const NbrArrays& nb, Target& T, int j, float& drho,
-                                           float& ax, float& ay, float& az)
-{
-    const float4 xr = __ldg(nb.xr + j);
-    const float4 sa = __ldg(nb.sa + j);
-    const float4 sb = __ldg(nb.sb + j);
-    const float3 vj = kPk ? unpack_velocity(sb.z, sb.w) : make_float3(sb.z, sb.w, __ldg(nb.vz + j));
-    const float a[8] = {xr.x, xr.y, xr.z, 0.0f, vj.x, vj.y, vj.z, xr.w};
-    const float b[6] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y};
-    const float dx = T.x.x - a[0], dy = T.x.y - a[1], dz = T.x.z - a[2];
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float q = sqrt_approx(r2) * K.ih;
-    const float t = fmaxf(2.0f - q, 0.0f);
-    const float fac = K.Cg * t * t * t;
-    const float gx = fac * dx, gy = fac * dy, gz = fac * dz;
-    const float vx = T.v.x - a[4], vy = T.v.y - a[5], vz = T.v.z - a[6];
-    drho += vx * gx + vy * gy + vz * gz;
-    const float Txx = T.Sxx + b[0], Tyy = T.Syy + b[1], Tzz = T.Szz + b[2];
-    const float Txy = T.Sxy + b[3], Txz = T.Sxz + b[4], Tyz = T.Syz + b[5];
-    float px = Txx * gx + Txy * gy + Txz * gz;
-    float py = Txy * gx + Tyy * gy + Tyz * gz;
-    float pz = Txz * gx + Tyz * gy + Tzz * gz;
-    {
-        /* Pi = -alpha cs h vr / ((r^2 + eta) rhobar) for vr < 0 */
-        const float vr = fminf(vx * dx + vy * dy + vz * dz, 0.0f);
-        const float pi = __fdividef(-K.avc * K.h * vr, (r2 + K.eta) * (0.5f * (T.v.w + a[7])));
-        px -= pi * gx;
-        py -= pi * gy;
-        pz -= pi * gz;
-    }
-    if (kArtp) {
-        const float wk = K.Cw * t * t * t * t * (q + 0.5f);
-        const float f = __fdividef(wk, K.wdr);
-        const float f4 = (f * f) * (f * f);
-        const float Rjx = b[0] > 0.f ? -K.eps * b[0] : 0.f;
-        const float Rjy = b[1] > 0.f ? -K.eps * b[1] : 0.f;
-        const float Rjz = b[2] > 0.f ? -K.eps * b[2] : 0.f;
-        px += (T.Rx + Rjx) * f4 * gx;
-        py += (T.Ry + Rjy) * f4 * gy;
-        pz += (T.Rz + Rjz) * f4 * gz;
-    }
-    ax += px;
-    ay += py;
-    az += pz;
-    const float Vj = K.m * __fdividef(1.0f, a[7]);
-    const float wx = Vj * vx, wy = Vj * vy, wz = Vj * vz;
-    T.l00 -= wx * gx; T.l01 -= wx * gy; T.l02 -= wx * gz;
-    T.l10 -= wy * gx; T.l11 -= wy * gy; T.l12 -= wy * gz;
-    T.l20 -= wz * gx; T.l21 -= wz * gy; T.l22 -= wz * gz;
 }
 
 /* One pair into T's sums.  kKahan selects the mixed form: the density
@@ -262,32 +274,52 @@ __device__ __forceinline__ void pair_terms(const PairConst& K, const NbrArrays& 
 template <bool kKahan = false>
 __device__ __forceinline__ void pair_body_rec(const PairConst& K, const NbrArrays& nb, Target& T, int j)
 {
+    PackedRecord<kKahan> r;
+    load_record(nb, j, r);
+    float d = 0.f, x = 0.f, y = 0.f, z = 0.f;
+    if (K.artp)
+        pair_terms<true>(K, r, T, d, x, y, z);
+    else
+        pair_terms<false>(K, r, T, d, x, y, z);
     if (kKahan) {
-        float d = 0.f, x = 0.f, y = 0.f, z = 0.f;
-        if (K.artp)
-            pair_terms<true, true>(K, nb, T, j, d, x, y, z);
-        else
-            pair_terms<false, true>(K, nb, T, j, d, x, y, z);
         kahan_add(T.drho, T.cdrho, d);
         kahan_add(T.ax, T.cax, x);
         kahan_add(T.ay, T.cay, y);
         kahan_add(T.az, T.caz, z);
-    } else if (K.artp) {
-        pair_terms<true, false>(K, nb, T, j, T.drho, T.ax, T.ay, T.az);
     } else {
-        pair_terms<false, false>(K, nb, T, j, T.drho, T.ax, T.ay, T.az);
+        T.drho += d;
+        T.ax += x;
+        T.ay += y;
+        T.az += z;
     }
+}
+
+/* The target's rates from its sums: acceleration and density rate, spin and
+ * strain rate. */
+struct TargetRates {
+    float4 a, w;
+    tensor2d de;
+};
+
+__device__ __forceinline__ TargetRates rates_of(const Parameters* __restrict__ P, const PairConst& K, const Target& T)
+{
+    const float c = K.mCg, hc = 0.5f * K.mCg;
+    TargetRates r;
+    r.a = make_float4(fmaf(c, T.ax, __ldg(&P->acc_x)), fmaf(c, T.ay, __ldg(&P->acc_y)), fmaf(c, T.az, __ldg(&P->acc_z)),
+                      c * T.drho);
+    r.w = make_float4(hc * (T.l10 - T.l01), hc * (T.l20 - T.l02), hc * (T.l21 - T.l12), 0.0f);
+    r.de = make_tensor2d(c * T.l00, c * T.l11, c * T.l22, hc * (T.l01 + T.l10), hc * (T.l02 + T.l20),
+                         hc * (T.l12 + T.l21));
+    return r;
 }
 
 __device__ __forceinline__ void store_rates(const Parameters* __restrict__ P, const PairConst& K, const Rates& rt,
                                             int i, const Target& T)
 {
-    rt.accad[i] = make_float4(K.m * T.ax + __ldg(&P->acc_x), K.m * T.ay + __ldg(&P->acc_y),
-                              K.m * T.az + __ldg(&P->acc_z), K.m * T.drho);
-    rt.spin[i] = make_float4(0.5f * (T.l10 - T.l01), 0.5f * (T.l20 - T.l02), 0.5f * (T.l21 - T.l12), 0.0f);
-    store_t2(rt.acestn, i,
-             make_tensor2d(T.l00, T.l11, T.l22, 0.5f * (T.l01 + T.l10), 0.5f * (T.l02 + T.l20),
-                           0.5f * (T.l12 + T.l21)));
+    const TargetRates r = rates_of(P, K, T);
+    rt.accad[i] = r.a;
+    rt.spin[i] = r.w;
+    store_t2(rt.acestn, i, r.de);
 }
 
 /* The 27-cell walk of one particle (both layers), calling f(j) for every
@@ -450,6 +482,10 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
     }
     flush();
     if (active) {
+        /* the list's last group of four filled up with the target itself
+         * (the split build's lists are filled up by their renewal) */
+        if (!kSplit)
+            for (int k = ni; k < LQ_NBR_CAP && (k & 3); ++k) list[(size_t)k * stride + t] = i;
         count_out[t] = ni;
         if (kSplit) shell_count[t] = ns;
         if ((ni > LQ_NBR_CAP || ns > LQ_NBR_CAP) && health) atomicAdd(health + HEALTH_NBR_OVERFLOW, 1);
@@ -471,7 +507,7 @@ __global__ void __launch_bounds__(kBlock) k_pack_neighbors(int first, int np, St
     }
     const float4 x = __ldg(st.pos + i);
     const float4 v = __ldg(st.vel + i);
-    nb.xr[o] = make_float4(x.x, x.y, x.z, v.w);
+    nb.xs[2 * (size_t)o] = make_float4(x.x, x.y, x.z, v.w);
     store_packed<kPk>(nb, o, v, load_t2(st.str, i));
 }
 
@@ -547,47 +583,121 @@ __global__ void __launch_bounds__(kBlock) k_list_refresh(int first, int ntarget,
             }
         }
     }
+    for (int k = n; k < LQ_NBR_CAP && (k & 3); ++k) list[(size_t)k * stride + t] = i;
     count[t] = n;
     if (n > LQ_NBR_CAP && health) atomicAdd(health + HEALTH_NBR_OVERFLOW, 1);
 }
 
-/* The sums over one target's list (entry k at p[k * stride]), four
- * entries per group, the next group's entries fetched ahead so the
- * dependent neighbour loads do not wait on the list stream.  The last
- * group is filled up with the target itself (exact zeros), so a group has
- * no branch.  The compensated (mixed) form adds each group's plain sum of
+/* Each target's list put into an order in which the lanes of a warp gather
+ * from different banks.  The pair kernel's lanes take consecutive targets,
+ * and row k of their lists is one gather per lane: eight lanes form one
+ * pass over the banks when their records' slots differ modulo 8 (eight
+ * 16-byte words per 128 bytes), and as many passes as the fullest residue
+ * holds otherwise.  In the order of the cell walk the residues are as good
+ * as random: about 26 passes for the two gathers of a warp's row, 12 being
+ * the least.  Target t takes an entry of residue (t + k) mod 8 in row k
+ * while it has one, else of the next residue that it has: about 16 (counted
+ * on the cylinder's lists; with the gathers in separate 16-byte words the
+ * launch went from 703 to 646 us at 1.97 M targets).  It pays where lists
+ * last: a build costs 1.8 ms there and this pass 0.5, the two pair launches
+ * of each of the 20 to 80 steps between builds gain 0.1 ms.
+ *
+ * One thread per target.  Its entries (kArrangeRows at a time) stand in
+ * shared memory as one chain per residue (hd: the chain's first row, nxt:
+ * the row after each), then leave in the rows' order.  Bound by the two
+ * passes over the list rows and the chains' shared-memory latency.  A list
+ * that overflowed is left as it is. */
+constexpr int kArrangeRows = 96;    /* an ordinary list (about 80 entries) in one piece; 7 blocks per SM */
+constexpr int kArrangeBlock = 64;
+__global__ void __launch_bounds__(kArrangeBlock) k_list_arrange(int ntarget, const int* __restrict__ count, int* list,
+                                                                int stride)
+{
+    __shared__ int ent[kArrangeRows][kArrangeBlock];
+    __shared__ unsigned char nxt[kArrangeRows][kArrangeBlock], hd[8][kArrangeBlock];
+    const int t = blockIdx.x * kArrangeBlock + threadIdx.x, x = threadIdx.x;
+    if (t >= ntarget) return;
+    const int n = __ldg(count + t);
+    if (n > LQ_NBR_CAP) return;
+    for (int base = 0; base < n; base += kArrangeRows) {
+        const int m = min(n - base, kArrangeRows);
+        int* p = list + (size_t)base * stride + t;
+        unsigned have = 0;      /* bit r: residue r's chain has entries */
+#pragma unroll 8
+        for (int k = 0; k < m; ++k) {
+            const int j = p[(size_t)k * stride], r = j & 7;
+            ent[k][x] = j;
+            nxt[k][x] = (have >> r & 1u) ? hd[r][x] : (unsigned char)255;
+            hd[r][x] = (unsigned char)k;
+            have |= 1u << r;
+        }
+        int k = 0;
+        /* while every chain has an entry: eight rows at a time, one from each */
+        for (const int w = t + base; k + 8 <= m && have == 255u; k += 8) {
+            int row[8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) row[o] = hd[(w + o) & 7][x];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                const unsigned char next = nxt[row[o]][x];
+                p[(size_t)(k + o) * stride] = ent[row[o]][x];
+                hd[(w + o) & 7][x] = next;
+                if (next == 255) have &= ~(1u << ((w + o) & 7));
+            }
+        }
+        for (; k < m; ++k) {
+            const int w = (t + base + k) & 7;
+            const int r = (w + __ffs((int)((have | have << 8) >> w)) - 1) & 7;
+            const int row = hd[r][x];
+            const unsigned char next = nxt[row][x];
+            p[(size_t)k * stride] = ent[row][x];
+            hd[r][x] = next;
+            if (next == 255) have &= ~(1u << r);
+        }
+    }
+}
+
+/* The sums over one target's list (entry k at p[k * stride]), in groups of
+ * four entries; the list's builder has filled the last group up with the
+ * target itself (exact zeros), so a group has no branch and no test.  A
+ * group's four records are gathered together and the next group's entries
+ * are fetched a group ahead, so the dependent gathers do not wait on the
+ * list stream.  The compensated (mixed) form adds each group's plain sum of
  * four pairs to the compensated sums and reads the packed velocity. */
 template <bool kKahan, bool kArtp>
 __device__ __forceinline__ void list_sums(const PairConst& K, const NbrArrays& nb, Target& T, const int* p, int n,
                                           int stride, int i, int np)
 {
     const size_t step4 = 4 * (size_t)stride;
-    int nxt[4];
+    auto entry = [&](int u) {
+        const int j = ld_list(p + (size_t)u * stride);
+        return lq_in_range(j, np) ? j : i;
+    };
+    if (n <= 0) return;
+    int cur[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) nxt[u] = u < n ? ld_list(p + u * stride) : i;
+    for (int u = 0; u < 4; ++u) cur[u] = entry(u);
     for (int k = 0; k < n; k += 4) {
-        p += step4;
-        int cur[4];
+        if (k + 4 < n) p += step4;      /* the last group fetches its own entries again */
+        int nxt[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            cur[u] = nxt[u];
-            nxt[u] = k + 4 + u < n ? ld_list(p + u * stride) : i;
-        }
+        for (int u = 0; u < 4; ++u) nxt[u] = entry(u);
+        PackedRecord<kKahan> r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) load_record(nb, cur[u], r[u]);
         if (kKahan) {
             float d = 0.f, x = 0.f, y = 0.f, z = 0.f;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (lq_in_range(cur[u], np)) pair_terms<kArtp, true>(K, nb, T, cur[u], d, x, y, z);
+            for (int u = 0; u < 4; ++u) pair_terms<kArtp>(K, r[u], T, d, x, y, z);
             kahan_add(T.drho, T.cdrho, d);
             kahan_add(T.ax, T.cax, x);
             kahan_add(T.ay, T.cay, y);
             kahan_add(T.az, T.caz, z);
         } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (lq_in_range(cur[u], np))
-                    pair_terms<kArtp, false>(K, nb, T, cur[u], T.drho, T.ax, T.ay, T.az);
+            for (int u = 0; u < 4; ++u) pair_terms<kArtp>(K, r[u], T, T.drho, T.ax, T.ay, T.az);
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
     }
 }
 
@@ -932,8 +1042,7 @@ __global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameter
         float2 sb[kG];
 #pragma unroll
         for (int u = 0; u < kG; ++u) {
-            xr[u] = __ldg(nb.xr + j[u]);
-            sa[u] = __ldg(nb.sa + j[u]);
+            load_xs(nb, j[u], xr[u], sa[u]);
             sb[u] = __ldg(reinterpret_cast<const float2*>(nb.sb + j[u]));
         }
 #pragma unroll
@@ -1003,11 +1112,11 @@ __device__ __forceinline__ void filter_groups(const NbrArrays& nb, const int* p,
         float2 sb[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            xr[u] = __ldg(nb.xr + j[u]);
             if (kStress) {
-                sa[u] = __ldg(nb.sa + j[u]);
+                load_xs(nb, j[u], xr[u], sa[u]);
                 sb[u] = __ldg(reinterpret_cast<const float2*>(nb.sb + j[u]));
             } else {
+                xr[u] = __ldg(nb.xs + 2 * (size_t)j[u]);
                 sa[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 sb[u] = make_float2(0.f, 0.f);
             }
@@ -1164,13 +1273,13 @@ const int kPairShapes[kPairShapeCount][3] = {{kBlock, LQ_PAIR_MIN_BLOCKS, 0},
                                              {128, -32, 0},
                                              {768, 1, 1},
                                              {384, 2, 1},
-                                             {640, 1, 1},
+                                             {256, 3, 1},
                                              {320, 2, 1}};
 
-/* The native driver's launch shape before any tuning: the tiled 640 x 1
- * shape once the targets fill at least four waves of 640-thread blocks on
- * every SM, the 128-thread shape 0 below that (a small case would leave
- * SMs idle with large blocks). */
+/* The native driver's launch shape before any tuning: the tiled 256 x 3
+ * shape from 2560 targets per SM on, the 128-thread shape 0 below that (a
+ * small case leaves SMs idle at the end of a tiled launch: 230 k targets,
+ * plain form, 92 us with shape 0 and 99 with 256 x 3 tiled). */
 int default_pair_shape(int npm)
 {
     int dev = 0, sms = 0;
@@ -1179,7 +1288,7 @@ int default_pair_shape(int npm)
         cudaGetLastError();
         return 0;
     }
-    return (long long)npm >= 4LL * sms * kPairShapes[kDefaultTiledShape][0] ? kDefaultTiledShape : 0;
+    return (long long)npm >= 2560LL * sms ? kDefaultTiledShape : 0;
 }
 
 /* Tile height (cells) for a block of `threads` targets: a 3 x 3-column
@@ -1281,6 +1390,15 @@ int launch_neighbor_list_range(const Parameters* ph, const Parameters* pd, int f
     return LQ_OK;
 }
 
+int launch_list_arrange(int n, const NeighborList& nl, cudaStream_t s)
+{
+    if (n <= 0) return LQ_OK;
+    if (nl.stride < n) return set_error(LQ_ERR_ARG, "list order: stride %d < targets %d", nl.stride, n);
+    k_list_arrange<<<blocks_for(n, kArrangeBlock), kArrangeBlock, 0, s>>>(n, nl.count, nl.list, nl.stride);
+    LQ_TRY_CUDA(cudaGetLastError(), "k_list_arrange");
+    return LQ_OK;
+}
+
 int launch_pack_neighbors(const Parameters* ph, const State& st, float* rec, int first, cudaStream_t s,
                           bool packed_velocity, const int* map)
 {
@@ -1364,8 +1482,8 @@ int launch_interaction_list(const Parameters* ph, const Parameters* pd, const St
 {
     if (ph->npm <= 0) return LQ_OK;
     if (rec) {
-        if (reinterpret_cast<uintptr_t>(rec) % 16 != 0)
-            return set_error(LQ_ERR_ARG, "interaction: packed neighbour arrays must be 16-byte aligned");
+        if (reinterpret_cast<uintptr_t>(rec) % 32 != 0)
+            return set_error(LQ_ERR_ARG, "interaction: packed neighbour arrays must be 32-byte aligned");
         const NbrArrays nb = nbr_arrays(rec, ph->np);
         if (rows && (!map || !pack || shape == 5 || shape == 6))
             return set_error(LQ_ERR_ARG, "interaction: list rows need a record map, a pack and a thread-per-target "
@@ -1382,7 +1500,7 @@ int launch_interaction_list(const Parameters* ph, const Parameters* pd, const St
         switch (shape) {
             case 7: LQ_PAIR_LAUNCH(768, 1); break;
             case 8: LQ_PAIR_LAUNCH(384, 2); break;
-            case 9: LQ_PAIR_LAUNCH(640, 1); break;
+            case 9: LQ_PAIR_LAUNCH(256, 3); break;
             case 10: LQ_PAIR_LAUNCH(320, 2); break;
             case 1: LQ_PAIR_LAUNCH(64, 12); break;
             case 2: LQ_PAIR_LAUNCH(256, 3); break;
