@@ -15,6 +15,7 @@
 
 #include "lq_internal.cuh"
 #include "lq_device.cuh"
+#include "lq_integrate.cuh"
 #include <predictor_corrector.h>
 
 namespace lqb {
@@ -22,9 +23,9 @@ namespace lqb {
 namespace {
 
 constexpr int kBlock = 128;
-/* resident blocks per SM asked of the model-3 instantiations: 4 caps them at
- * 128 registers (a few spilled bytes), measured faster than 1 (168 registers)
- * and 6 (80) on the 2.85 M-particle slope */
+/* resident blocks per SM asked of the model-3 kernels: 4 caps them at 128
+ * registers; on the 2.85 M-particle slope in flow the two integrations take
+ * 1299 us a step with 4, 1332 with 5 (96 registers, spills), 1348 with 6 */
 #ifndef LQ_VW_MIN_BLOCKS
 #define LQ_VW_MIN_BLOCKS 4
 #endif
@@ -40,58 +41,135 @@ constexpr int kBlock = 128;
 
 inline int blocks_for(long long n, int b) { return (int)((n + b - 1) / b); }
 
-/* FP64 position (pressure p in the float word's w) and velocity into the
- * float high words x, v and, with `lo`, the low words of `out` at slot i. */
-__device__ __forceinline__ void split_words(const State& out, int i, const double4& xd, const double4& vd, float p,
-                                            float4& x, float4& v, bool lo = true)
+/* What the model-3 kernels store of a finished stress: the stress, the void
+ * ratio (`full`: not in a stage buffer), the packed entry's stress words,
+ * and a non-finite stress in health unless the slot's kinematics already
+ * counted. */
+__device__ __forceinline__ void store_vw(const State& out, int i, const T6d& sd, double e, bool full,
+                                         const NbrArrays& nb, int* __restrict__ health)
 {
-    float4 xl, vl;
-    split4(make_double4(xd.x, xd.y, xd.z, 0.0), x, xl);
-    split4(vd, v, vl);
-    x.w = p;
-    if (lo) {
-        out.xlo[i] = xl;
-        out.vlo[i] = vl;
+    const tensor2d s = narrow6(sd);
+    store_t2(out.str, i, s);
+    if (full) reinterpret_cast<float*>(out.idep + i)[2] = (float)e;
+    const float4 v = out.vel[i];
+    if (nb.xs) store_packed_stress(nb, i, v.w, s);
+    if (health && !finite_stress(s) && finite_kinematics(out.pos[i], v)) atomicAdd(health + HEALTH_NONFINITE, 1);
+}
+
+/* Model 3: the stress and void ratio of the material slots over part x dt,
+ * by the first trial sub-step, which spans the whole interval.  Nine in ten
+ * particles of a half step and two in three of a full step need no more
+ * (the slope in flow); the others are queued with the step of their next
+ * trial, for k_vw_finish.  A kernel of its own, after the kinematics, keeps
+ * the trial's state in as few registers as its two rate evaluations allow:
+ * it is bound by FP64 latency, so by the warps in flight (the FP64 pipe is
+ * busy 46 % of the time at 15 warps per SM).  On the 2.85 M-particle slope
+ * a half step's trials take 258 us and its queue 138, a full step's 271 and
+ * 330; one kernel that ran each particle to its end took 660 and 740 with
+ * the kinematics (106 and 177) in it. */
+__global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_trial(const Parameters* __restrict__ P, double part,
+                                                                       int npb, int np, const float4* idep,
+                                                                       const tensor2d* src_str, State out, bool full,
+                                                                       Rates rt, MaterialTable vw, NbrArrays nb,
+                                                                       int* __restrict__ health, SubstepQueue q)
+{
+    const int i = npb + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= np) return;
+    const double dt = part * (double)__ldg(&P->dt);
+    const float4 id = idep[i];
+    const tensor2d s0 = load_t2_rw(src_str, i);
+    if (!(dt > 0.0)) {
+        store_vw(out, i, widen6(s0), id.z, full, nb, health);
+        return;
+    }
+    const VWConst& c = *vw_row(vw, id.x);
+    VWTrial g;
+    const float4 w = __ldg(rt.spin + i);
+    const tensor2d de = load_t2(rt.acestn, i);
+    if (g.run(c, dt, s0, id.z, de, w)) {
+        store_vw(out, i, g.s, g.e, full, nb, health);
+        return;
+    }
+    const bool hard = !(g.h > 0.2 * dt);    /* the largest cut of a step: the longest runs */
+    const unsigned act = __activemask();
+    const unsigned hards = __ballot_sync(act, hard);
+    const unsigned peers = hard ? hards : act & ~hards;
+    const int lane = threadIdx.x & 31, leader = __ffs((int)peers) - 1;
+    int at = 0;
+    if (lane == leader) at = atomicAdd(q.counts + (hard ? 0 : 1), __popc(peers));
+    at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
+    if (!hard) at = q.cap - 1 - at;
+    q.item[at] = i;
+    q.h[at] = g.h;
+}
+
+/* Model 3: the queued particles' remaining sub-steps from the start of
+ * their interval (src_str, and the void ratio in idep).  The numbers of sub-steps
+ * differ widely between neighbours (a warp of the slope's full steps needs
+ * ten for its slowest lane, two on average), so a lane that has finished
+ * takes the next particle of the queue while the others go on: every lane
+ * evaluates a rate in every turn.  The particles whose step was cut most
+ * come first, since the longest chain of evaluations ends the launch.
+ * Bound by FP64 latency, and in small cases by the longest chain: 64
+ * trials of two evaluations take 150 us. */
+__global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_finish(const Parameters* __restrict__ P, double part,
+                                                                        const float4* idep,
+                                                                        const tensor2d* src_str, State out,
+                                                                        bool full, Rates rt, MaterialTable vw,
+                                                                        NbrArrays nb, int* __restrict__ health,
+                                                                        SubstepQueue q)
+{
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int nhard = q.counts[0], n = nhard + q.counts[1];
+    const double dt = part * (double)__ldg(&P->dt);
+    int i = -1;
+    bool drained = false;
+    VWIntegration g{};
+    const VWConst* c = nullptr;
+    tensor2d de{};
+    float4 w{};
+    for (;;) {
+        const unsigned idle = __ballot_sync(FULL, i < 0 && !drained);
+        if (idle) {
+            int at = 0;
+            if (lane == __ffs((int)idle) - 1) at = atomicAdd(q.counts + 2, __popc(idle));
+            at = __shfl_sync(FULL, at, __ffs((int)idle) - 1) + __popc(idle & ((1u << lane) - 1u));
+            if (idle >> lane & 1u) {
+                if (at < n) {
+                    if (at >= nhard) at = q.cap - 1 - (at - nhard);
+                    i = q.item[at];
+                    const float4 id = idep[i];
+                    c = vw_row(vw, id.x);
+                    w = __ldg(rt.spin + i);
+                    de = load_t2(rt.acestn, i);
+                    g.start(widen6(load_t2_rw(src_str, i)), id.z, de, q.h[at], 1);
+                } else {
+                    drained = true;
+                }
+            }
+        }
+        if (__all_sync(FULL, i < 0)) break;
+        if (i >= 0 && !g.advance(*c, dt, de, w)) {
+            store_vw(out, i, g.s, g.e, full, nb, health);
+            i = -1;
+        }
     }
 }
 
-/* The same, storing the high words too. */
-__device__ __forceinline__ void store_split(const State& out, int i, const double4& xd, const double4& vd, float p,
-                                            bool lo = true)
+__global__ void k_vw_rows(int n, const float* __restrict__ rows, VWConst* __restrict__ derived)
 {
-    float4 x, v;
-    split_words(out, i, xd, vd, p, x, v, lo);
-    out.pos[i] = x;
-    out.vel[i] = v;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) derived[k] = vw_const(rows + 10 * (size_t)k);
 }
 
-/* A material slot's entry of the pair kernel's packed neighbour arrays from
- * the position, velocity and stress just stored (what k_pack_neighbors
- * would write from them), when nb is set: the native driver's integrators
- * pack the slots they update, so a stage needs no pack of its own.  kPk
- * (the mixed form) packs the velocity into two words. */
-template <bool kPk>
-__device__ __forceinline__ void pack_slot(const NbrArrays& nb, int i, const float4& x, const float4& v,
-                                          const tensor2d& s)
-{
-    if (!nb.xs) return;
-    nb.xs[2 * (size_t)i] = make_float4(x.x, x.y, x.z, v.w);
-    store_packed<kPk>(nb, i, v, s);
-}
-
-/* Half step of the material slots (reference src/predictor_corrector.cu:169-218):
- * v += dt/2 a; rho += dt/2 drho; x += dt/2 v_new; eps += dt/2 deps;
- * stress and plastic strain from the model at dt/2.  With `stage` the
- * output is a stage buffer that only the neighbour kernels and the
- * corrector read: the position and velocity high words (with the
- * pressure), the object word and the stress; the corrector restarts the
- * strain, the plastic strain and the FP64 kinematics from its snapshot, so
- * the strain (neither read nor written), the low words and, for the
- * hypoplastic model, the plastic strain are left out. */
-template <bool kMixed, bool kVW>
-__global__ void __launch_bounds__(kBlock, kVW ? LQ_VW_MIN_BLOCKS : LQ_INT_MIN_BLOCKS) k_predict(const Parameters* __restrict__ P, int np, int npb, State in,
-                                                    State out, State snap, bool do_snap, Rates rt, MaterialTable mt,
-                                                    MaterialTable vw, NbrArrays nb, bool stage)
+/* Predictor of the slots, into `out` (or in place); with do_snap each
+ * slot's state is copied to `snap` first. */
+template <bool kMixed>
+__global__ void __launch_bounds__(kBlock, LQ_INT_MIN_BLOCKS) k_predict(const Parameters* __restrict__ P, int np,
+                                                                       int npb, State in, State out, State snap,
+                                                                       bool do_snap, Rates rt, MaterialTable mt,
+                                                                       NbrArrays nb, bool stage)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
@@ -116,310 +194,107 @@ __global__ void __launch_bounds__(kBlock, kVW ? LQ_VW_MIN_BLOCKS : LQ_INT_MIN_BL
         if (out.pos != in.pos) store_t2(out.str, i, s0);
         return;
     }
-    const float dt = __ldg(&P->dt);
-    const Material M = particle_material(load_material(P), mt, id.x);
-    const float4 a = __ldg(rt.accad + i);
-    const float4 w = __ldg(rt.spin + i);
-    const tensor2d de = load_t2(rt.acestn, i);
-
-    if (kMixed) {
-        /* FP64 accumulation of velocity, density and position; FP64 stress update */
-        const double hdt = 0.5 * (double)dt;
-        double4 vd = join4(v0, in.vlo[i]), xd = join4(x0, in.xlo[i]);
-        vd.x += hdt * a.x; vd.y += hdt * a.y; vd.z += hdt * a.z; vd.w += hdt * a.w;
-        xd.x += hdt * vd.x; xd.y += hdt * vd.y; xd.z += hdt * vd.z;
-        T6d e = widen6(e0), dd = widen6(de);
-        e.xx += dd.xx * hdt; e.yy += dd.yy * hdt; e.zz += dd.zz * hdt;
-        e.xy += dd.xy * hdt; e.xz += dd.xz * hdt; e.yz += dd.yz * hdt;
-        double p = x0.w, ep = id.y, ev = id.z;
-        T6d sd = widen6(s0);
-        if (kVW) {
-            /* the kinematics are stored before the sub-stepping, whose FP64
-             * registers then need not share the SM with them */
-            store_split(out, i, xd, vd, x0.w, !stage);
-            if (!stage) store_t2(out.stn, i, narrow6(e));
-            const float epf = stage ? id.y : (float)sqrt(2.0 / 3.0 * contract6(e, e));
-            vw_update_d(vw_const(vw, id.x), hdt, de, w, sd, ev);
-            out.idep[i] = make_float4(id.x, epf, (float)ev, id.w);
-            const tensor2d sn = narrow6(sd);
-            store_t2(out.str, i, sn);
-            pack_slot<kMixed>(nb, i, out.pos[i], out.vel[i], sn);   /* kinematics stored above */
-            return;
-        }
-        if (M.model == 1) {
-            dp_update_d(M, hdt, w, dd, p, ep, sd);
-        } else {
-            hypo_update_d(M, hdt, dd, w, sd);
-            if (!stage) ep = sqrt(2.0 / 3.0 * contract6(e, e));
-        }
-        float4 xh, vh;
-        split_words(out, i, xd, vd, (float)p, xh, vh, !stage);
-        out.pos[i] = xh;
-        out.vel[i] = vh;
-        out.idep[i] = make_float4(id.x, (float)ep, (float)ev, id.w);
-        const tensor2d sn = narrow6(sd);
-        store_t2(out.str, i, sn);
-        if (!stage) store_t2(out.stn, i, narrow6(e));
-        pack_slot<kMixed>(nb, i, xh, vh, sn);
-        return;
-    }
-    float4 v = v0;
-    v.x += 0.5f * dt * a.x;
-    v.y += 0.5f * dt * a.y;
-    v.z += 0.5f * dt * a.z;
-    v.w += 0.5f * dt * a.w;
-    float4 x = x0;
-    x.x += 0.5f * dt * v.x;
-    x.y += 0.5f * dt * v.y;
-    x.z += 0.5f * dt * v.z;
-    const tensor2d e = e0 + de * (0.5f * dt);
-
-    float p = x0.w;
-    float ep = id.y, ev = id.z;
-    tensor2d s = s0;
-    if (kVW) {
-        /* the adaptive sub-stepping runs in FP64 in both forms; the
-         * kinematics are stored first */
-        out.pos[i] = x;
-        out.vel[i] = v;
-        if (!stage) store_t2(out.stn, i, e);
-        const float epf = stage ? id.y : sqrtf(2.0f / 3.0f * J2(e));
-        T6d sd = widen6(s0);
-        double evd = ev;
-        vw_update_d(vw_const(vw, id.x), 0.5 * (double)dt, de, w, sd, evd);
-        out.idep[i] = make_float4(id.x, epf, (float)evd, id.w);
-        const tensor2d sn = narrow6(sd);
-        store_t2(out.str, i, sn);
-        pack_slot<kMixed>(nb, i, out.pos[i], out.vel[i], sn);   /* kinematics stored above */
-        return;
-    }
-    if (M.model == 1) {
-        dp_update(M, 0.5f * dt, w, de, p, ep, s);
-    } else {
-        hypo_update(M, 0.5f * dt, de, w, s);
-        if (!stage) ep = sqrtf(2.0f / 3.0f * J2(e));
-    }
-    x.w = p;
-    out.pos[i] = x;
-    out.vel[i] = v;
-    out.idep[i] = make_float4(id.x, ep, ev, id.w);
-    store_t2(out.str, i, s);
-    if (!stage) store_t2(out.stn, i, e);
-    pack_slot<kMixed>(nb, i, x, v, s);
+    predict_slot<kMixed>(P, i, in, out, load_rates(rt, i), mt, nb, stage, x0, v0, id, s0, e0);
 }
 
-/* Full step from the snapshot (reference src/predictor_corrector.cu:256-307):
- * v = v0 + dt a; x = x0 + dt/2 (v + v0); eps = eps0 + dt deps; the model
- * restarts from the snapshot stress and plastic strain; the pressure passed
- * in is the current one.  Reads the current state `cur` and the snapshot
- * `ini` (at ini_idx[i], or i), writes `out` (which may be `cur` or `ini`).
- * When out differs from cur, boundary slots are copied from cur (their
- * stress is the latest Adami extrapolation).  With `verlet`, each material
- * particle also checks whether neighbour lists built at positions xbuild
- * stay valid through the next step: it raises *rebuild when twice its
- * displacement plus a bound on its next step's motion reaches the skin. */
-struct VerletCheck {
-    const float4* xbuild;
-    int* rebuild;
-    float half_skin;
-    float dt_bound;   /* the largest step the next one can take */
-    const float4* xwide;   /* two-level lists: positions at the wide build */
-    float half_margin;     /* (wide - skin) / 2 */
-};
-
-/* The list checks of one material particle at its new position x. */
-__device__ __forceinline__ void verlet_check(const VerletCheck& vc, int i, const float4& x, const float4& v,
-                                             const float4& a)
-{
-    const float4 xb = __ldg(vc.xbuild + i);
-    const float dx = x.x - xb.x, dy = x.y - xb.y, dz = x.z - xb.z;
-    const float moved = sqrtf(dx * dx + dy * dy + dz * dz);
-    const float speed = sqrtf(v.x * v.x + v.y * v.y + v.z * v.z);
-    const float accel = sqrtf(a.x * a.x + a.y * a.y + a.z * a.z);
-    /* next step: the predictor half step and the corrector full step
-     * move a particle by at most dt |v| + dt^2 |a| each; 2x covers both */
-    const float dtb = vc.dt_bound;
-    const float ahead = 2.0f * dtb * (speed + dtb * accel);
-    if (!(moved + ahead < vc.half_skin)) atomicOr(vc.rebuild, 1);
-    if (vc.xwide) {
-        /* lists renewed at x from the wide ones hold every pair within
-         * 2h + skin while no particle is (wide - skin) / 2 from xwide */
-        const float4 xw = __ldg(vc.xwide + i);
-        const float ex = x.x - xw.x, ey = x.y - xw.y, ez = x.z - xw.z;
-        if (!(sqrtf(ex * ex + ey * ey + ez * ez) < vc.half_margin)) atomicOr(vc.rebuild, 2);
-    }
-}
-
-template <bool kMixed, bool kVW>
-__global__ void __launch_bounds__(kBlock, kVW ? LQ_VW_MIN_BLOCKS : LQ_INT_MIN_BLOCKS) k_correct(const Parameters* __restrict__ P, int np, int npb, State cur,
-                                                    State ini, const int* __restrict__ ini_idx, State out, Rates rt,
-                                                    int* __restrict__ health, VerletCheck verlet, int first,
-                                                    MaterialTable mt, MaterialTable vw, NbrArrays nb)
+/* Corrector of the material slots from the snapshot `ini` (at ini_idx[i],
+ * or i) and the current state `cur` into `out` (which may be either). */
+template <bool kMixed>
+__global__ void __launch_bounds__(kBlock, LQ_INT_MIN_BLOCKS) k_correct(const Parameters* __restrict__ P, int np,
+                                                                       int npb, State cur, State ini,
+                                                                       const int* __restrict__ ini_idx, State out,
+                                                                       Rates rt, int* __restrict__ health,
+                                                                       VerletCheck verlet, int first,
+                                                                       MaterialTable mt, NbrArrays nb)
 {
     const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     if (i < npb) return;    /* boundary slots: Adami writes both buffers */
     const int k = ini_idx ? __ldg(ini_idx + i) : i;
-    const float dt = __ldg(&P->dt);
-    const float4 a = __ldg(rt.accad + i);
-    const float4 w = __ldg(rt.spin + i);
-    const tensor2d de = load_t2(rt.acestn, i);
-    const float4 x0 = ini.pos[k];
-    const float4 v0 = ini.vel[k];
-    const float4 id0 = ini.idep[k];
-    const float ep0 = id0.y;
-    const tensor2d s0 = load_t2_rw(ini.str, k);
-    const tensor2d e0 = load_t2_rw(ini.stn, k);
-    const float4 xc = cur.pos[i];
-    const float4 id = cur.idep[i];
-    const Material M = particle_material(load_material(P), mt, id.x);
-
-    if (kVW) {
-        /* model 3: the kinematics, the health of the kinematics and the
-         * Verlet check come before the FP64 sub-stepping, so that its
-         * registers need not share the SM with them */
-        float4 v, x;
-        tensor2d e;
-        float ep;
-        if (kMixed) {
-            const double ddt = dt;
-            const double4 v0d = join4(v0, ini.vlo[k]), x0d = join4(x0, ini.xlo[k]);
-            double4 vd, xd;
-            vd.x = v0d.x + ddt * a.x; vd.y = v0d.y + ddt * a.y; vd.z = v0d.z + ddt * a.z; vd.w = v0d.w + ddt * a.w;
-            xd.x = 0.5 * (vd.x + v0d.x) * ddt + x0d.x;
-            xd.y = 0.5 * (vd.y + v0d.y) * ddt + x0d.y;
-            xd.z = 0.5 * (vd.z + v0d.z) * ddt + x0d.z;
-            xd.w = 0.0;
-            T6d ed = widen6(e0);
-            const T6d dd = widen6(de);
-            ed.xx += dd.xx * ddt; ed.yy += dd.yy * ddt; ed.zz += dd.zz * ddt;
-            ed.xy += dd.xy * ddt; ed.xz += dd.xz * ddt; ed.yz += dd.yz * ddt;
-            split_words(out, i, xd, vd, xc.w, x, v);
-            e = narrow6(ed);
-            ep = (float)sqrt(2.0 / 3.0 * contract6(ed, ed));
-        } else {
-            v.x = v0.x + dt * a.x;
-            v.y = v0.y + dt * a.y;
-            v.z = v0.z + dt * a.z;
-            v.w = v0.w + dt * a.w;
-            x.x = 0.5f * (v.x + v0.x) * dt + x0.x;
-            x.y = 0.5f * (v.y + v0.y) * dt + x0.y;
-            x.z = 0.5f * (v.z + v0.z) * dt + x0.z;
-            x.w = xc.w;
-            e = e0 + de * dt;
-            ep = sqrtf(2.0f / 3.0f * J2(e));
-        }
-        out.pos[i] = x;
-        out.vel[i] = v;
-        store_t2(out.stn, i, e);
-        const bool bad = !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(v.x) && isfinite(v.y) &&
-                           isfinite(v.z) && isfinite(v.w));
-        if (verlet.xbuild) verlet_check(verlet, i, x, v, a);
-        T6d sd = widen6(s0);
-        double evd = id0.z;
-        vw_update_d(vw_const(vw, id.x), (double)dt, de, w, sd, evd);
-        const tensor2d s = narrow6(sd);
-        out.idep[i] = make_float4(id.x, ep, (float)evd, id.w);
-        store_t2(out.str, i, s);
-        pack_slot<kMixed>(nb, i, out.pos[i], out.vel[i], s);   /* kinematics stored above */
-        if (health && (bad || !(isfinite(s.xx) && isfinite(s.yy) && isfinite(s.zz) && isfinite(s.xy) &&
-                                isfinite(s.xz) && isfinite(s.yz))))
-            atomicAdd(health + HEALTH_NONFINITE, 1);
-        return;
-    }
-    float4 v, x;
-    tensor2d s, e;
-    float ep, ev = id.z;
-    if (kMixed) {
-        const double ddt = dt;
-        const double4 v0d = join4(v0, ini.vlo[k]), x0d = join4(x0, ini.xlo[k]);
-        double4 vd, xd;
-        vd.x = v0d.x + ddt * a.x; vd.y = v0d.y + ddt * a.y; vd.z = v0d.z + ddt * a.z; vd.w = v0d.w + ddt * a.w;
-        xd.x = 0.5 * (vd.x + v0d.x) * ddt + x0d.x;
-        xd.y = 0.5 * (vd.y + v0d.y) * ddt + x0d.y;
-        xd.z = 0.5 * (vd.z + v0d.z) * ddt + x0d.z;
-        xd.w = 0.0;
-        T6d ed = widen6(e0), dd = widen6(de);
-        ed.xx += dd.xx * ddt; ed.yy += dd.yy * ddt; ed.zz += dd.zz * ddt;
-        ed.xy += dd.xy * ddt; ed.xz += dd.xz * ddt; ed.yz += dd.yz * ddt;
-        double pd = xc.w, epd = ep0;
-        T6d sd = widen6(s0);
-        if (M.model == 1) {
-            dp_update_d(M, ddt, w, dd, pd, epd, sd);
-        } else {
-            hypo_update_d(M, ddt, dd, w, sd);
-            epd = sqrt(2.0 / 3.0 * contract6(ed, ed));
-        }
-        split_words(out, i, xd, vd, (float)pd, x, v);
-        s = narrow6(sd);
-        e = narrow6(ed);
-        ep = (float)epd;
-    } else {
-        v.x = v0.x + dt * a.x;
-        v.y = v0.y + dt * a.y;
-        v.z = v0.z + dt * a.z;
-        v.w = v0.w + dt * a.w;
-        x.x = 0.5f * (v.x + v0.x) * dt + x0.x;
-        x.y = 0.5f * (v.y + v0.y) * dt + x0.y;
-        x.z = 0.5f * (v.z + v0.z) * dt + x0.z;
-        e = e0 + de * dt;
-        float p = xc.w;
-        ep = ep0;
-        s = s0;
-        if (M.model == 1) {
-            dp_update(M, dt, w, de, p, ep, s);
-        } else {
-            hypo_update(M, dt, de, w, s);
-            ep = sqrtf(2.0f / 3.0f * J2(e));
-        }
-        x.w = p;
-    }
-    out.pos[i] = x;
-    out.vel[i] = v;
-    out.idep[i] = make_float4(id.x, ep, ev, id.w);
-    store_t2(out.str, i, s);
-    store_t2(out.stn, i, e);
-    pack_slot<kMixed>(nb, i, x, v, s);
-    if (health) {
-        const bool ok = isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(v.x) && isfinite(v.y) &&
-                        isfinite(v.z) && isfinite(v.w) && isfinite(s.xx) && isfinite(s.yy) && isfinite(s.zz) &&
-                        isfinite(s.xy) && isfinite(s.xz) && isfinite(s.yz);
-        if (!ok) atomicAdd(health + HEALTH_NONFINITE, 1);
-    }
-    if (verlet.xbuild) verlet_check(verlet, i, x, v, a);
+    correct_slot<kMixed>(P, i, k, cur.pos[i].w, cur.idep[i], ini, out, load_rates(rt, i), mt, nb, health, verlet);
 }
 
 }  // namespace
 
+size_t vw_row_bytes() { return sizeof(VWConst); }
+
+int launch_vw_rows(const MaterialTable& vw, void* derived, cudaStream_t s)
+{
+    if (vw.n <= 0) return LQ_OK;
+    k_vw_rows<<<blocks_for(vw.n, kBlock), kBlock, 0, s>>>(vw.n, vw.p, static_cast<VWConst*>(derived));
+    LQ_TRY_CUDA(cudaGetLastError(), "k_vw_rows");
+    return LQ_OK;
+}
+
+namespace {
+
+/* The stresses of the material slots over part x dt: every slot's first
+ * trial, then the queued ones by as many blocks as the device holds. */
+int enqueue_substeps(const Parameters* ph, const Parameters* pd, double part, const float4* idep,
+                     const tensor2d* src_str, const State& out, bool full, const Rates& r, const MaterialTable& vw,
+                     const NbrArrays& nb, int* health, const SubstepQueue& q, cudaStream_t s)
+{
+    int dev = 0, sms = 0;
+    LQ_TRY_CUDA(cudaGetDevice(&dev), "sub-steps");
+    LQ_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "sub-steps");
+    LQ_TRY_CUDA(cudaMemsetAsync(q.counts, 0, 3 * sizeof(int), s), "sub-step queue");
+    k_vw_trial<<<blocks_for(ph->npm, kBlock), kBlock, 0, s>>>(pd, part, ph->npb, ph->np, idep, src_str, out, full, r,
+                                                              vw, nb, health, q);
+    LQ_TRY_CUDA(cudaGetLastError(), "k_vw_trial");
+    k_vw_finish<<<sms * LQ_VW_MIN_BLOCKS, kBlock, 0, s>>>(pd, part, idep, src_str, out, full, r, vw, nb, health, q);
+    LQ_TRY_CUDA(cudaGetLastError(), "k_vw_finish");
+    return LQ_OK;
+}
+
+}  // namespace
+
+int check_substeps(const Parameters* ph, const char* who, const MaterialTable& vw, const SubstepQueue& q)
+{
+    if (ph->constitutive_model != 3) return LQ_OK;
+    if (!vw.p || vw.n <= 0 || !vw.derived)
+        return set_error(LQ_ERR_ARG, "%s: constitutive model 3 needs a von Wolffersdorff table", who);
+    if (!q.item || !q.h || !q.counts || q.cap < ph->npm)
+        return set_error(LQ_ERR_ARG, "%s: constitutive model 3 needs a sub-step queue", who);
+    return LQ_OK;
+}
+
+int launch_predict_substeps(const Parameters* ph, const Parameters* pd, const State& in, const State& out,
+                            const Rates& r, cudaStream_t s, const MaterialTable& vw, float* rec,
+                            const SubstepQueue& q)
+{
+    if (ph->constitutive_model != 3 || ph->npm <= 0) return LQ_OK;
+    const NbrArrays nb = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
+    return enqueue_substeps(ph, pd, 0.5, in.idep, in.str, out, false, r, vw, nb, nullptr, q, s);
+}
+
+int launch_correct_substeps(const Parameters* ph, const Parameters* pd, const State& st, const Rates& r, int* health,
+                            cudaStream_t s, const MaterialTable& vw, float* rec, const SubstepQueue& q)
+{
+    if (ph->constitutive_model != 3 || ph->npm <= 0) return LQ_OK;
+    const NbrArrays nb = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
+    return enqueue_substeps(ph, pd, 1.0, st.idep, st.str, st, true, r, vw, nb, health, q, s);
+}
+
 int launch_predict(const Parameters* ph, const Parameters* pd, const State& in, const State& out, const State* snap,
                    const Rates& r, cudaStream_t s, const MaterialTable& mt, const MaterialTable& vw, float* rec,
-                   bool stage)
+                   bool stage, const SubstepQueue& q)
 {
     if (ph->np <= 0) return LQ_OK;
-    if (ph->constitutive_model == 3 && (!vw.p || vw.n <= 0))
-        return set_error(LQ_ERR_ARG, "predictor: constitutive model 3 needs a von Wolffersdorff table");
+    LQ_TRY(check_substeps(ph, "predictor", vw, q));
     const bool do_snap = snap && snap->pos;
     if (stage && (do_snap || out.pos == in.pos))
         return set_error(LQ_ERR_ARG, "predictor: a stage buffer needs its own output and no snapshot");
+    if (ph->constitutive_model == 3 && !stage)
+        return set_error(LQ_ERR_ARG, "predictor: constitutive model 3 runs in stage buffers only");
     State sn = do_snap ? *snap : State{nullptr, nullptr, nullptr, nullptr, nullptr};
-    /* model 3 gets its own instantiation: its FP64 sub-stepping needs far
-     * more registers than the other models' kernels */
-    const bool vwm = ph->constitutive_model == 3;
     const int nb = blocks_for(ph->np, kBlock);
     const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
-    if (in.xlo && out.xlo) {
-        if (vwm) k_predict<true, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, vw, pk,
-                                                              stage);
-        else k_predict<true, false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, vw, pk,
-                                                              stage);
-    } else {
-        if (vwm) k_predict<false, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, vw, pk,
-                                                              stage);
-        else k_predict<false, false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, vw, pk,
-                                                              stage);
-    }
+    if (in.xlo && out.xlo)
+        k_predict<true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, pk, stage);
+    else
+        k_predict<false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, in, out, sn, do_snap, r, mt, pk, stage);
     LQ_TRY_CUDA(cudaGetLastError(), "k_predict");
-    return LQ_OK;
+    return launch_predict_substeps(ph, pd, in, out, r, s, vw, rec, q);
 }
 
 int launch_correct(const Parameters* ph, const Parameters* pd, const State& cur, const State& ini,
@@ -428,40 +303,32 @@ int launch_correct(const Parameters* ph, const Parameters* pd, const State& cur,
     if (ph->npm <= 0) return LQ_OK;
     if (ph->constitutive_model == 3)
         return set_error(LQ_ERR_ARG, "corrector: constitutive model 3 needs a von Wolffersdorff table");
-    k_correct<false, false><<<blocks_for(ph->npm, kBlock), kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, ini_idx, cur, r, health,
-                                                             VerletCheck{nullptr, nullptr, 0.0f, 0.0f, nullptr, 0.0f}, ph->npb,
-                                                             MaterialTable(), MaterialTable(),
-                                                             NbrArrays{nullptr, nullptr, nullptr});
+    k_correct<false><<<blocks_for(ph->npm, kBlock), kBlock, 0, s>>>(
+        pd, ph->np, ph->npb, cur, ini, ini_idx, cur, r, health, VerletCheck{nullptr, nullptr, 0.0f, 0.0f, nullptr, 0.0f},
+        ph->npb, MaterialTable(), NbrArrays{nullptr, nullptr, nullptr});
     LQ_TRY_CUDA(cudaGetLastError(), "k_correct");
     return LQ_OK;
 }
 
 int launch_correct_into(const Parameters* ph, const Parameters* pd, const State& cur, const State& ini,
-                        const State& out, const Rates& r, int* health, const float4* xbuild, int* rebuild,
-                        float skin, cudaStream_t s, const MaterialTable& mt, const MaterialTable& vw,
-                        const float4* xwide, float wide, float* rec)
+                        const Rates& r, int* health, const ListCheck& lists, cudaStream_t s, const MaterialTable& mt,
+                        const MaterialTable& vw, float* rec, const SubstepQueue& q)
 {
-    if (ph->np <= 0) return LQ_OK;
-    if (ph->constitutive_model == 3 && (!vw.p || vw.n <= 0))
-        return set_error(LQ_ERR_ARG, "corrector: constitutive model 3 needs a von Wolffersdorff table");
-    /* a dynamic step never exceeds the fixed one, cfl h / cs (ph->dt) */
-    if (xwide && !(wide > skin)) return set_error(LQ_ERR_ARG, "corrector: the wide cut-off must exceed the skin");
-    const VerletCheck vc{xbuild, rebuild, 0.5f * skin, ph->dt, xwide, 0.5f * (wide - skin)};
-    const bool vwm = ph->constitutive_model == 3;
     if (ph->npm <= 0) return LQ_OK;
+    LQ_TRY(check_substeps(ph, "corrector", vw, q));
+    if (lists.xwide && !(lists.wide > lists.skin))
+        return set_error(LQ_ERR_ARG, "corrector: the wide cut-off must exceed the skin");
+    const VerletCheck vc = verlet_of(ph, lists);
     /* material slots only: boundary slots are written by Adami into both
      * buffers */
     const int nb = blocks_for(ph->npm, kBlock), f = ph->npb;
     const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
-    if (cur.xlo && ini.xlo && out.xlo) {
-        if (vwm) k_correct<true, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);
-        else k_correct<true, false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);
-    } else {
-        if (vwm) k_correct<false, true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);
-        else k_correct<false, false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, out, r, health, vc, f, mt, vw, pk);
-    }
+    if (ini.xlo)
+        k_correct<true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, ini, r, health, vc, f, mt, pk);
+    else
+        k_correct<false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, ini, r, health, vc, f, mt, pk);
     LQ_TRY_CUDA(cudaGetLastError(), "k_correct");
-    return LQ_OK;
+    return launch_correct_substeps(ph, pd, ini, r, health, s, vw, rec, q);
 }
 
 }  // namespace lqb

@@ -381,17 +381,15 @@ __device__ __forceinline__ void hypo_update_d(const Material& M, double dtp, con
  * principal direction) the deviator of That is scaled back to
  * tan psi = sqrt2 (1 - 1e-3) at the same mean stress. */
 struct VWConst {
-    double a, a2, fbk, lnhs, ihs, n, ed0, ec0, lnec0, ei0, alpha, beta, tol;
+    double a, a2, fbk, lnhs, n, ed0, ec0, lnec0, ei0, alpha, beta, tol;
     int maxsub;
 };
 
-/* Row constants; the powers of constants are formed once here:
+/* The constants of one table row; the powers of constants are formed here,
+ * once per row when the table is set (k_vw_rows):
  * fbk = (hs / n) (ei0 / ec0)^beta / (3 + a^2 - a sqrt3 ((ei0 - ed0) / (ec0 - ed0))^alpha). */
-__device__ __forceinline__ VWConst vw_const(const MaterialTable& mt, float id)
+__device__ __forceinline__ VWConst vw_const(const float* r)
 {
-    int k = (int)id;
-    k = k < 0 ? 0 : (k >= mt.n ? mt.n - 1 : k);
-    const float* r = mt.p + 10 * k;
     VWConst c;
     const double phic = (double)__ldg(r) * 3.14159265358979323846 / 180.0;
     const double sphi = sin(phic);
@@ -407,11 +405,18 @@ __device__ __forceinline__ VWConst vw_const(const MaterialTable& mt, float id)
     c.tol = __ldg(r + 8);
     c.maxsub = (int)__ldg(r + 9);
     c.lnhs = log(hs);
-    c.ihs = 1.0 / hs;
     c.lnec0 = log(c.ec0);
     const double den = 3.0 + c.a2 - c.a * sqrt(3.0) * pow((c.ei0 - c.ed0) / (c.ec0 - c.ed0), c.alpha);
     c.fbk = (hs / c.n) * pow(c.ei0 / c.ec0, c.beta) / den;
     return c;
+}
+
+/* The derived row of object id `id` (rows out of range are clamped). */
+__device__ __forceinline__ const VWConst* vw_row(const MaterialTable& mt, float id)
+{
+    int k = (int)id;
+    k = k < 0 ? 0 : (k >= mt.n ? mt.n - 1 : k);
+    return static_cast<const VWConst*>(mt.derived) + k;
 }
 
 __device__ __forceinline__ double trace_cube6(const T6d& A)
@@ -421,12 +426,19 @@ __device__ __forceinline__ double trace_cube6(const T6d& A)
            6.0 * A.xy * A.xz * A.yz;
 }
 
-/* The rate with the state-dependent powers through shared logarithms:
- * pr = -trT/hs, pr^n = exp(n ln pr), pr^(1-n) = pr / pr^n, ex = exp(-pr^n),
- * fe = exp(beta (ln ec0 - pr^n - ln e)), fd = exp(alpha ln((e - ed) / (ec - ed))).
- * The stretching d stays in float (it is read as float) and the deviator
- * That* is formed from That where needed, to spare registers. */
-__device__ __forceinline__ void vw_rate_d(const VWConst& c, const T6d& Tin, double e, const tensor2d& d,
+/* The rate with the state-dependent powers through shared logarithms,
+ * pr = -trT/hs, pr^n = exp(n ln pr), ex = exp(-pr^n),
+ * pr^(1-n) fe = exp((1 - n) ln pr + beta (ln ec0 - pr^n - ln e)),
+ * fd = exp(alpha ln((e - ed) / (ec - ed))), and with few quotients: FP64
+ * divisions and roots are chains of a dozen dependent operations, and the
+ * sub-stepping is bound by such chains.  The three quotients by That:That,
+ * ei and ec - ed share one reciprocal, and
+ * tan psi cos 3theta = -sqrt18 tr(That*^3) / (That*:That*) enters F's
+ * quotient multiplied out (limited to |tan psi|, as cos 3theta to 1).
+ * The stretching d stays in float (it is read as float), its norm nD is
+ * formed once per integration, and the deviator That* is formed from That
+ * where needed, to spare registers. */
+__device__ __forceinline__ void vw_rate_d(const VWConst& c, const T6d& Tin, double e, const tensor2d& d, double nD,
                                           const float4& w, T6d& R, double& edot)
 {
     T6d Th = Tin;
@@ -442,7 +454,7 @@ __device__ __forceinline__ void vw_rate_d(const VWConst& c, const T6d& Tin, doub
     double sxx = Th.xx - third, syy = Th.yy - third, szz = Th.zz - third;
     double TsTs = sxx * sxx + syy * syy + szz * szz + 2.0 * (Th.xy * Th.xy + Th.xz * Th.xz + Th.yz * Th.yz);
     double tpsi = sqrt(3.0 * TsTs);
-    const double lim = sqrt(2.0) * (1.0 - 1e-3);
+    const double lim = 1.4142135623730951 * (1.0 - 1e-3);
     if (tpsi > lim) {
         const double f = lim / tpsi;
         sxx *= f; syy *= f; szz *= f;
@@ -451,26 +463,25 @@ __device__ __forceinline__ void vw_rate_d(const VWConst& c, const T6d& Tin, doub
         tpsi = lim;
     }
     const double ThTh = contract6(Th, Th);
-    double c3t = 1.0;
+    const double t2 = tpsi * tpsi;
+    double num = 2.0 - t2, den = 2.0 + 1.4142135623730951 * tpsi;   /* cos 3theta = 1 on the hydrostatic axis */
     if (TsTs > 1e-30) {
-        const T6d Ts{sxx, syy, szz, Th.xy, Th.xz, Th.yz};
-        c3t = -sqrt(6.0) * trace_cube6(Ts) / (TsTs * sqrt(TsTs));
+        const double tc = -4.2426406871192851 * trace_cube6(T6d{sxx, syy, szz, Th.xy, Th.xz, Th.yz});
+        num *= TsTs;
+        den = 2.0 * TsTs + 1.4142135623730951 * fmax(-tpsi * TsTs, fmin(tpsi * TsTs, tc));
     }
-    c3t = fmax(-1.0, fmin(1.0, c3t));
-    const double F = sqrt(fmax(tpsi * tpsi / 8.0 + (2.0 - tpsi * tpsi) / (2.0 + sqrt(2.0) * tpsi * c3t), 0.0)) -
-                     tpsi / (2.0 * sqrt(2.0));
+    const double F = sqrt(fmax(0.125 * t2 + num / den, 0.0)) - 0.35355339059327379 * tpsi;
     const double lnpr = log(-trT) - c.lnhs;
     const double prn = exp(c.n * lnpr);
     const double ex = exp(-prn);
-    const double ei = c.ei0 * ex, ec = c.ec0 * ex, ed = c.ed0 * ex;
-    const double fe = exp(c.beta * (c.lnec0 - prn - log(e)));
-    const double q = (e - ed) / (ec - ed);
+    const double ei = c.ei0 * ex, ed = c.ed0 * ex, ecd = c.ec0 * ex - ed;
+    const double fpe = exp((1.0 - c.n) * lnpr + c.beta * (c.lnec0 - prn - log(e)));
+    const double rcp = 1.0 / (ThTh * ei * ecd);
+    const double q = (e - ed) * (rcp * ThTh * ei);
     const double fd = q > 0.0 ? exp(c.alpha * log(q)) : (c.alpha == 0.0 ? 1.0 : 0.0);
-    const double fb = c.fbk * (1.0 + 1.0 / ei) * (-trT * c.ihs) / prn;
     const double dxx = d.xx, dyy = d.yy, dzz = d.zz, dxy = d.xy, dxz = d.xz, dyz = d.yz;
     const double ThD = Th.xx * dxx + Th.yy * dyy + Th.zz * dzz + 2.0 * (Th.xy * dxy + Th.xz * dxz + Th.yz * dyz);
-    const double nD = sqrt(dxx * dxx + dyy * dyy + dzz * dzz + 2.0 * (dxy * dxy + dxz * dxz + dyz * dyz));
-    const double k0 = fb * fe / ThTh;
+    const double k0 = c.fbk * (1.0 + rcp * ThTh * ecd) * fpe * (rcp * ei * ecd);
     const double F2 = F * F, nf = fd * c.a * F * nD;
     const T6d J = jaumann_d(w, Tin);
     R.xx = k0 * (F2 * dxx + c.a2 * Th.xx * ThD + nf * (Th.xx + sxx)) + J.xx;
@@ -482,24 +493,38 @@ __device__ __forceinline__ void vw_rate_d(const VWConst& c, const T6d& Tin, doub
     edot = (1.0 + e) * (dxx + dyy + dzz);
 }
 
-/* Adaptive explicit integration over dt; returns the number of sub-steps.
- * The loop has one rate evaluation site (inlined once): each pass evaluates
- * either the first rate k1 of a trial at (s, e) or the second, k2, at the
- * Euler point s + h k1.  The Heun result is s + h/2 (k1 + k2) and its
- * difference from the Euler point, h/2 (k2 - k1), is the error estimate; a
- * rejected trial keeps its k1. */
-__device__ __forceinline__ int vw_update_d(const VWConst& c, double dt, const tensor2d& d, const float4& w, T6d& s,
-                                           double& e)
-{
-    double t = 0.0, h = dt;
-    int steps = 0;
-    T6d k1{}, x = s;
-    double ke1 = 0.0, xe = e;
-    bool have_k1 = false;
-    while (t < dt) {
+/* Adaptive explicit integration of (s, e) over dt, one rate evaluation per
+ * call of advance: the first rate k1 of a trial at (s, e), or the second,
+ * k2, at the Euler point s + h k1.  The Heun result is s + h/2 (k1 + k2)
+ * and its difference from the Euler point, h/2 (k2 - k1), is the error
+ * estimate; a rejected trial keeps its k1.  Evaluations are counted in
+ * trials (`steps`); the last one allowed spans the rest of the interval. */
+struct VWIntegration {
+    T6d s, k1, x;
+    double e, ke1, xe, t, h, nD;
+    int steps;
+    bool have_k1;
+
+    /* From the state (s0, e0) under the stretching d, the next trial over
+     * h0 and `done` trials already rejected at that state. */
+    __device__ __forceinline__ void start(const T6d& s0, double e0, const tensor2d& d, double h0, int done)
+    {
+        const T6d dd = widen6(d);
+        nD = sqrt(contract6(dd, dd));
+        s = x = s0;
+        e = xe = e0;
+        t = 0.0;
+        h = h0;
+        steps = done;
+        have_k1 = false;
+    }
+
+    /* One rate evaluation; false once t reaches dt. */
+    __device__ __forceinline__ bool advance(const VWConst& c, double dt, const tensor2d& d, const float4& w)
+    {
         T6d r;
         double re;
-        vw_rate_d(c, x, xe, d, w, r, re);
+        vw_rate_d(c, x, xe, d, nD, w, r, re);
         if (!have_k1) {
             k1 = r;
             ke1 = re;
@@ -514,15 +539,15 @@ __device__ __forceinline__ int vw_update_d(const VWConst& c, double dt, const te
             ++steps;
             const bool last = steps >= c.maxsub - 1 || h <= dt * 1e-6;
             if (err <= c.tol || last) {
-                s = s2;
+                s = x = s2;
                 e += hh * (ke1 + re);
+                xe = e;
                 t += h;
+                if (!(t < dt)) return false;
                 const double g = err > 0.0 ? 0.9 * sqrt(c.tol / err) : 2.0;
                 h *= fmin(2.0, fmax(0.2, g));
                 have_k1 = false;
-                x = s;
-                xe = e;
-                continue;
+                return true;
             }
             h *= fmax(0.2, 0.9 * sqrt(c.tol / err));
         }
@@ -532,9 +557,47 @@ __device__ __forceinline__ int vw_update_d(const VWConst& c, double dt, const te
         x = T6d{s.xx + h * k1.xx, s.yy + h * k1.yy, s.zz + h * k1.zz, s.xy + h * k1.xy, s.xz + h * k1.xz,
                 s.yz + h * k1.yz};
         xe = e + h * ke1;
+        return true;
     }
-    return steps;
-}
+};
+
+/* The first trial of an integration, over the whole interval: the same
+ * arithmetic as VWIntegration's first two calls of advance, with the start
+ * kept in float (it is read as float) while the second rate is formed. */
+struct VWTrial {
+    T6d s;          /* the result */
+    double e, h;    /* its void ratio; the next trial's step when rejected */
+
+    /* True when the trial is accepted (or the last allowed). */
+    __device__ __forceinline__ bool run(const VWConst& c, double dt, const tensor2d& s0, double e0, const tensor2d& d,
+                                        const float4& w)
+    {
+        const T6d dd = widen6(d);
+        const double nD = sqrt(contract6(dd, dd));
+        T6d k1{}, r, x = widen6(s0);
+        double ke1 = 0.0, re, xe = e0;
+#pragma unroll 1
+        for (int pass = 0;; ++pass) {
+            vw_rate_d(c, x, xe, d, nD, w, r, re);
+            if (pass) break;
+            k1 = r;
+            ke1 = re;
+            x = T6d{s0.xx + dt * r.xx, s0.yy + dt * r.yy, s0.zz + dt * r.zz, s0.xy + dt * r.xy, s0.xz + dt * r.xz,
+                    s0.yz + dt * r.yz};
+            xe = e0 + dt * re;
+        }
+        const double hh = 0.5 * dt;
+        s = T6d{s0.xx + hh * (k1.xx + r.xx), s0.yy + hh * (k1.yy + r.yy), s0.zz + hh * (k1.zz + r.zz),
+                s0.xy + hh * (k1.xy + r.xy), s0.xz + hh * (k1.xz + r.xz), s0.yz + hh * (k1.yz + r.yz)};
+        const T6d df{hh * (r.xx - k1.xx), hh * (r.yy - k1.yy), hh * (r.zz - k1.zz),
+                     hh * (r.xy - k1.xy), hh * (r.xz - k1.xz), hh * (r.yz - k1.yz)};
+        const double err = sqrt(contract6(df, df) / fmax(contract6(s, s), 1e-30));
+        e = e0 + hh * (ke1 + re);
+        if (err <= c.tol || c.maxsub <= 2) return true;
+        h = dt * fmax(0.2, 0.9 * sqrt(c.tol / err));
+        return false;
+    }
+};
 
 /* Packed neighbour data for the list pair kernel: dense arrays over all
  * slots, with s = sigma / rho^2,

@@ -70,6 +70,18 @@ struct Cells {
 struct MaterialTable {
     const float* p = nullptr;
     int n = 0;
+    const void* derived = nullptr;   /* model 3: the rows' derived constants (launch_vw_rows) */
+};
+
+/* Model 3: the particles whose first trial sub-step was rejected, with the
+ * step their next trial takes (cap entries each): counts[0] whose step was
+ * cut most from the front, counts[1] others from the back; counts[2] is a
+ * cursor over both. */
+struct SubstepQueue {
+    int* item = nullptr;
+    double* h = nullptr;
+    int* counts = nullptr;
+    int cap = 0;
 };
 
 /* Per-object cell frames: when rows is set, a particle with object id k
@@ -227,24 +239,47 @@ int launch_shepard(const Parameters* par_host, const Parameters* par_dev, const 
  * its hypoplastic plastic strain are not written. */
 int launch_predict(const Parameters* par_host, const Parameters* par_dev, const State& in, const State& out,
                    const State* snap, const Rates& r, cudaStream_t s, const MaterialTable& mt = MaterialTable(),
-                   const MaterialTable& vw = MaterialTable(), float* rec = nullptr, bool stage = false);
+                   const MaterialTable& vw = MaterialTable(), float* rec = nullptr, bool stage = false,
+                   const SubstepQueue& q = SubstepQueue());
 /* Corrector in place on `cur`; ini values read at ini_idx[i] (identity when
  * ini_idx is null).  Non-finite results are counted in health. */
 int launch_correct(const Parameters* par_host, const Parameters* par_dev, const State& cur, const State& ini,
                    const int* ini_idx, const Rates& r, int* health, cudaStream_t s);
 
-/* Corrector from snapshot `ini` and current `cur` into `out`, material
- * slots only (boundary slots must already be the same in all three);
- * material particles raise bit 1 of *rebuild when neighbour
- * lists built at xbuild with this skin may not hold through the next step,
- * and (with xwide) bit 2 when a particle has moved (wide - skin) / 2 or
- * more from xwide, where lists with cut-off 2h + wide were built: lists
- * renewed from those now could miss a pair. */
+/* What the native corrector checks the neighbour lists against: positions
+ * at their build (skin) and, with two-level lists, at the wide build. */
+struct ListCheck {
+    const float4* xbuild = nullptr;
+    int* flag = nullptr;
+    float skin = 0.0f;
+    const float4* xwide = nullptr;
+    float wide = 0.0f;
+};
+
+/* Corrector from the snapshot `ini` and the current stage buffer `cur` into
+ * `ini`, material slots only; material particles raise bit 1 of *flag when
+ * neighbour lists built at xbuild with this skin may not hold through the
+ * next step, and (with xwide) bit 2 when a particle has moved
+ * (wide - skin) / 2 or more from xwide, where lists with cut-off 2h + wide
+ * were built: lists renewed from those now could miss a pair. */
 int launch_correct_into(const Parameters* par_host, const Parameters* par_dev, const State& cur, const State& ini,
-                        const State& out, const Rates& r, int* health, const float4* xbuild, int* rebuild,
-                        float skin, cudaStream_t s, const MaterialTable& mt = MaterialTable(),
-                        const MaterialTable& vw = MaterialTable(), const float4* xwide = nullptr,
-                        float wide = 0.0f, float* rec = nullptr);
+                        const Rates& r, int* health, const ListCheck& lists, cudaStream_t s,
+                        const MaterialTable& mt = MaterialTable(), const MaterialTable& vw = MaterialTable(),
+                        float* rec = nullptr, const SubstepQueue& q = SubstepQueue());
+/* Model 3's stresses after a stage's kinematics (nothing for the other
+ * models): the half step from `in` into the stage buffer `out`, the full
+ * step in place; r holds the spin and strain rates.  check_substeps: the
+ * table and queue that a model-3 launch needs. */
+int check_substeps(const Parameters* par_host, const char* who, const MaterialTable& vw, const SubstepQueue& q);
+int launch_predict_substeps(const Parameters* par_host, const Parameters* par_dev, const State& in, const State& out,
+                            const Rates& r, cudaStream_t s, const MaterialTable& vw, float* rec,
+                            const SubstepQueue& q);
+int launch_correct_substeps(const Parameters* par_host, const Parameters* par_dev, const State& st, const Rates& r,
+                            int* health, cudaStream_t s, const MaterialTable& vw, float* rec, const SubstepQueue& q);
+/* The derived constants of the n model-3 rows at vw.p (10 floats each) into
+ * `derived` (n x vw_row_bytes()); both integrators need them in vw.derived. */
+size_t vw_row_bytes();
+int launch_vw_rows(const MaterialTable& vw, void* derived, cudaStream_t s);
 
 /* List-driven Shepard filter (material targets and neighbours) reading
  * the neighbours from the packed records `rec` (required; the material

@@ -84,6 +84,7 @@ struct LqSim {
     int* host_flag = nullptr;          /* pinned mirror for the eager path */
     lqb::MaterialTable mt;             /* per-object materials (optional) */
     lqb::MaterialTable vw;             /* von Wolffersdorff rows (model 3) */
+    lqb::SubstepQueue subq;            /* particles with more than one sub-step (model 3) */
     float* rec = nullptr;              /* packed neighbour data, np x 13 floats */
     float* rho_f = nullptr;            /* density filter output (LQ_SIM_DENSITY_FILTER) */
     int pair_shape = 0;                /* launch shape of the pair kernel (lqb::kPairShapes) */
@@ -115,6 +116,11 @@ bool tiled(const LqSim* S) { return lqb::kPairShapes[S->pair_shape][2] != 0; }
 constexpr int kFlagLists = 1, kFlagSort = 2, kFlagAll = 3;
 
 bool two_level(const LqSim* S) { return S->wide > S->skin && S->wlm.list != nullptr; }
+
+lqb::ListCheck list_check(const LqSim* S)
+{
+    return lqb::ListCheck{S->xbuild, S->rebuild, S->skin, two_level(S) ? S->xwide : nullptr, S->wide};
+}
 
 /* Wide lists and their build positions, on first use of two-level lists. */
 int ensure_wide_lists(LqSim* S)
@@ -150,12 +156,13 @@ int ensure_tile_order(LqSim* S)
     return LQ_OK;
 }
 
-int alloc_state(LqSim* S, State& st)
+int alloc_state(LqSim* S, State& st, float4* idep = nullptr)
 {
     const size_t n = (size_t)S->np;
     LQ_TRY(dev_alloc(S, (void**)&st.pos, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&st.vel, n * sizeof(float4)));
-    LQ_TRY(dev_alloc(S, (void**)&st.idep, n * sizeof(float4)));
+    st.idep = idep;
+    if (!idep) LQ_TRY(dev_alloc(S, (void**)&st.idep, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&st.str, n * sizeof(tensor2d)));
     LQ_TRY(dev_alloc(S, (void**)&st.stn, n * sizeof(tensor2d)));
     if (S->flags & LQ_SIM_MIXED) {
@@ -193,7 +200,6 @@ __global__ void k_copy_state(int n, int npb, State in, State out, State out2, fl
     if (i < npb) {
         out2.pos[i] = in.pos[i];
         out2.vel[i] = in.vel[i];
-        out2.idep[i] = in.idep[i];
         const float2* a = reinterpret_cast<const float2*>(in.str) + 3 * (size_t)i;
         float2* b = reinterpret_cast<float2*>(out2.str) + 3 * (size_t)i;
         b[0] = a[0];
@@ -464,12 +470,12 @@ int enqueue_stages(LqSim* S, cudaStream_t s)
     /* predictor stage (reference src/loquat.cu:343-368) */
     LQ_TRY(enqueue_adami_pack(S, S->S, s));
     LQ_TRY(enqueue_interaction(S, S->S, s));
-    LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true));
+    LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true, S->subq));
     /* corrector stage (reference src/loquat.cu:371-396) */
     LQ_TRY(enqueue_adami_pack(S, S->S2, s));
     LQ_TRY(enqueue_interaction(S, S->S2, s));
-    LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->S, S->R, S->health, S->xbuild, S->rebuild, S->skin, s,
-                                    S->mt, S->vw, two_level(S) ? S->xwide : nullptr, S->wide, S->rec));
+    LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->R, S->health, list_check(S), s, S->mt, S->vw, S->rec,
+                                    S->subq));
     return enqueue_dynamic_dt(S, s);
 }
 
@@ -679,7 +685,7 @@ int create(LqSim* S, const Parameters* par, const float* pos, const float* vel, 
     LQ_TRY_CUDA(cudaMallocHost((void**)&S->host_flag, sizeof(int)), "pinned flag");
     LQ_TRY(dev_alloc(S, (void**)&S->pd, sizeof(Parameters)));
     LQ_TRY(alloc_state(S, S->S));
-    LQ_TRY(alloc_state(S, S->S2));
+    LQ_TRY(alloc_state(S, S->S2, S->S.idep));   /* the stage buffer shares the object words */
     LQ_TRY(alloc_state(S, S->T));
     const size_t n = (size_t)S->np;
     LQ_TRY(dev_alloc(S, (void**)&S->xbuild, n * sizeof(float4)));
@@ -968,8 +974,18 @@ extern "C" int lq_sim_set_hypoplastic(void* sim, int n, const float* table)
     float* d = nullptr;
     LQ_TRY(dev_alloc(S, (void**)&d, sizeof(float) * 10 * (size_t)n));
     LQ_TRY_CUDA(cudaMemcpy(d, table, sizeof(float) * 10 * (size_t)n, cudaMemcpyHostToDevice), "hypoplastic table");
+    void* derived = nullptr;
+    LQ_TRY(dev_alloc(S, &derived, lqb::vw_row_bytes() * (size_t)n));
+    if (!S->subq.item) {
+        LQ_TRY(dev_alloc(S, (void**)&S->subq.h, sizeof(double) * (size_t)S->np));
+        LQ_TRY(dev_alloc(S, (void**)&S->subq.counts, 3 * sizeof(int)));
+        LQ_TRY(dev_alloc(S, (void**)&S->subq.item, sizeof(int) * (size_t)S->np));
+        S->subq.cap = S->np;
+    }
+    LQ_TRY(lqb::launch_vw_rows(lqb::MaterialTable{d, n, nullptr}, derived, S->stream));
     S->vw.p = d;
     S->vw.n = n;
+    S->vw.derived = derived;
     S->vw_host.assign(table, table + 10 * (size_t)n);
     LQ_TRY(build_graphs(S));
     return LQ_OK;
@@ -1575,11 +1591,10 @@ int profiled_step(LqSim* S, PhaseTimer& T)
         LQ_TRY(T.close(s));
         LQ_TRY(T.mark(s, PH_INTEGRATE));
         if (stage == 0)
-            LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true));
+            LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true, S->subq));
         else {
-            LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->S, S->R, S->health, S->xbuild, S->rebuild,
-                                            S->skin, s, S->mt, S->vw, two_level(S) ? S->xwide : nullptr,
-                                            S->wide, S->rec));
+            LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->R, S->health, list_check(S), s, S->mt, S->vw,
+                                            S->rec, S->subq));
             LQ_TRY(enqueue_dynamic_dt(S, s));
         }
         LQ_TRY(T.close(s));
