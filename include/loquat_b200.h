@@ -306,8 +306,11 @@ int lq_sim_neighbor_entries(void* sim, long long* material, long long* boundary)
  * integrate, Shepard, neighbour-list build, renewal of two-level lists
  * (the phases of the reference's Timer, include/types.h:158-173, timed on
  * the device instead of with std::clock, with the search and the list
- * build and renewal split out).  phase_launches[8] (may be NULL) receives
- * how many times each phase ran. */
+ * build and renewal split out).  The thread-per-target pair shapes
+ * integrate their targets in the pair kernel: their steps count under
+ * interaction, and integrate holds what is left (model 3's stresses, the
+ * dynamic time step).  phase_launches[8] (may be NULL) receives how many
+ * times each phase ran. */
 int lq_sim_profile(void* sim, int nsteps, double* phase_ms, int* phase_launches);
 
 /* ---- XML / .dat formats (reference src/loquat_io.cu:69-370) ------------ */

@@ -160,6 +160,32 @@ struct NeighborList {
     int stride = 0;         /* >= npm, multiple of 32 */
 };
 
+/* What the native corrector checks the neighbour lists against: positions
+ * at their build (skin) and, with two-level lists, at the wide build. */
+struct ListCheck {
+    const float4* xbuild = nullptr;
+    int* flag = nullptr;
+    float skin = 0.0f;
+    const float4* xwide = nullptr;
+    float wide = 0.0f;
+};
+
+/* A stage of the native driver whose pair kernel integrates its targets:
+ * stage 1 takes the predictor step from `in` into the stage buffer `out`,
+ * stage 2 the corrector step of the snapshot `in` in place.  The new
+ * records go to rec_out (the stage that follows; not the arrays the pair
+ * kernel gathers from).  keep_rates stores the rates as well (the dynamic
+ * time step and model 3 read them). */
+struct StageOps {
+    int stage = 1;
+    State in{}, out{};
+    MaterialTable mt;
+    float* rec_out = nullptr;
+    int* health = nullptr;
+    ListCheck lists;
+    bool keep_rates = false;
+};
+
 /* ------------------------------------------------------------ operators */
 int launch_neighbor_list(const Parameters* par_host, const Parameters* par_dev, const float4* pos, const Cells& c,
                          const NeighborList& nl, cudaStream_t s);
@@ -175,20 +201,27 @@ int launch_neighbor_list(const Parameters* par_host, const Parameters* par_dev, 
 int launch_interaction_list(const Parameters* par_host, const Parameters* par_dev, const State& st, const Rates& r,
                             const Cells& c, const NeighborList& nl, cudaStream_t s, const Frames& fr = Frames(),
                             bool compensated = false, float* rec = nullptr, int shape = 0, bool pack = true,
-                            const int* order = nullptr, const int* rows = nullptr, const int* map = nullptr);
+                            const int* order = nullptr, const int* rows = nullptr, const int* map = nullptr,
+                            const StageOps* ops = nullptr);
+/* Whether a launch shape integrates its targets when asked to (ops); the
+ * warp-cooperative ones store their rates for the integrator kernels.  The
+ * thread-per-target shapes store rates in the plain form only. */
+bool integrates_in_pair_kernel(int shape);
 /* The packed neighbour arrays of slots [first, np) from the state;
- * packed_velocity selects the compensated pair kernel's record. */
+ * packed_velocity selects the compensated pair kernel's record.  The slots
+ * below n2 are packed into rec2 as well. */
 int launch_pack_neighbors(const Parameters* par_host, const State& st, float* rec, int first, cudaStream_t s,
-                          bool packed_velocity, const int* map = nullptr);
+                          bool packed_velocity, const int* map = nullptr, float* rec2 = nullptr, int n2 = 0);
 /* Adami over the boundary lists reading the packed arrays (material slots
  * packed), writing the boundary stress into the state, into str2 when set
  * and into the stress words of the packed arrays (the boundary slots'
- * other words, from the last full pack, stay).  With act / nact (device;
+ * other words, from the last full pack, stay), those of rec2 too when it is
+ * set.  With act / nact (device;
  * from launch_boundary_targets; act holds at least npb ints) only the
  * slots act[0 .. *nact) are visited. */
 int launch_adami_packed(const Parameters* par_host, const Parameters* par_dev, const State& st,
                         const NeighborList& nl, float* rec, cudaStream_t s, tensor2d* str2 = nullptr,
-                        const int* act = nullptr, const int* nact = nullptr);
+                        float* rec2 = nullptr, const int* act = nullptr, const int* nact = nullptr);
 /* The boundary slots t < npb with count[t] > 0 or count2[t] > 0 (count2
  * may be null), ascending, into act[0 .. *nact) on the device; temp holds
  * boundary_targets_temp_bytes(npb) bytes of scratch. */
@@ -245,16 +278,6 @@ int launch_predict(const Parameters* par_host, const Parameters* par_dev, const 
  * ini_idx is null).  Non-finite results are counted in health. */
 int launch_correct(const Parameters* par_host, const Parameters* par_dev, const State& cur, const State& ini,
                    const int* ini_idx, const Rates& r, int* health, cudaStream_t s);
-
-/* What the native corrector checks the neighbour lists against: positions
- * at their build (skin) and, with two-level lists, at the wide build. */
-struct ListCheck {
-    const float4* xbuild = nullptr;
-    int* flag = nullptr;
-    float skin = 0.0f;
-    const float4* xwide = nullptr;
-    float wide = 0.0f;
-};
 
 /* Corrector from the snapshot `ini` and the current stage buffer `cur` into
  * `ini`, material slots only; material particles raise bit 1 of *flag when

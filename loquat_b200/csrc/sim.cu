@@ -15,9 +15,11 @@
  *   per step (state in S, order fixed between rebuilds)
  *     [rebuild if flagged: search S, gather S -> T, copy T -> S, record the
  *      positions, build material and boundary lists]
- *     Adami(S), interaction(S), predictor S -> S2          (S is the snapshot)
- *     Adami(S2), interaction(S2), corrector (S2, S) -> S   (raises the flag)
- *     (Adami writes the boundary stress into S and S2; the integrators
+ *     Adami(S), interaction(S) with predictor S -> S2          (S is the snapshot)
+ *     Adami(S2), interaction(S2) with corrector (S2, S) -> S   (raises the flag)
+ *     (the thread-per-target pair kernels integrate each target as its sums
+ *     end; the warp-cooperative ones are followed by the integrator kernels;
+ *     Adami writes the boundary stress into S and S2; the integrators
  *     update the material slots only; S2 is a stage buffer: the predictor
  *     writes what the neighbour kernels and the corrector read from it,
  *     not its strain or low words)
@@ -85,7 +87,8 @@ struct LqSim {
     lqb::MaterialTable mt;             /* per-object materials (optional) */
     lqb::MaterialTable vw;             /* von Wolffersdorff rows (model 3) */
     lqb::SubstepQueue subq;            /* particles with more than one sub-step (model 3) */
-    float* rec = nullptr;              /* packed neighbour data, np x 13 floats */
+    float* rec = nullptr;              /* packed neighbour data of S, np x 13 floats */
+    float* rec2 = nullptr;             /* and of the stage buffer S2 */
     float* rho_f = nullptr;            /* density filter output (LQ_SIM_DENSITY_FILTER) */
     int pair_shape = 0;                /* launch shape of the pair kernel (lqb::kPairShapes) */
     lqb::TileOrder tile;               /* targets in tile order (tiled shapes; allocated on first use) */
@@ -389,12 +392,48 @@ int enqueue_renewal(LqSim* S, cudaStream_t s)
     return LQ_OK;
 }
 
-/* The pair sums of a stage in the current launch shape. */
-int enqueue_interaction(LqSim* S, const State& st, cudaStream_t s)
+/* The pair sums of a stage in the current launch shape; the
+ * thread-per-target shapes integrate each target with them. */
+int enqueue_interaction(LqSim* S, int stage, cudaStream_t s)
 {
     const lqb::Cells cells{S->g.start, nullptr, nullptr};
-    return lqb::launch_interaction_list(&S->ph, S->pd, st, S->R, cells, S->nlm, s, S->fr, S->flags & LQ_SIM_MIXED,
-                                        S->rec, S->pair_shape, false, tile_order(S));
+    const bool first = stage == 1;
+    lqb::StageOps ops;
+    ops.stage = stage;
+    ops.in = S->S;
+    ops.out = first ? S->S2 : S->S;
+    ops.mt = S->mt;
+    ops.rec_out = first ? S->rec2 : S->rec;
+    ops.health = first ? nullptr : S->health;
+    if (!first) ops.lists = list_check(S);
+    ops.keep_rates = !first && (S->flags & LQ_SIM_DYNAMIC_DT);
+    return lqb::launch_interaction_list(&S->ph, S->pd, first ? S->S : S->S2, S->R, cells, S->nlm, s, S->fr,
+                                        S->flags & LQ_SIM_MIXED, first ? S->rec : S->rec2, S->pair_shape, false,
+                                        tile_order(S), nullptr, nullptr,
+                                        lqb::integrates_in_pair_kernel(S->pair_shape) ? &ops : nullptr);
+}
+
+/* What is left of a stage's integration after its pair kernel: all of it
+ * with the warp-cooperative shapes, model 3's stresses with the others. */
+int enqueue_integration(LqSim* S, int stage, cudaStream_t s)
+{
+    const Parameters* ph = &S->ph;
+    const Parameters* pd = S->pd;
+    if (lqb::integrates_in_pair_kernel(S->pair_shape)) {
+        if (stage == 1) return lqb::launch_predict_substeps(ph, pd, S->S, S->S2, S->R, s, S->vw, S->rec2, S->subq);
+        return lqb::launch_correct_substeps(ph, pd, S->S, S->R, S->health, s, S->vw, S->rec, S->subq);
+    }
+    if (stage == 1)
+        return lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec2, true, S->subq);
+    return lqb::launch_correct_into(ph, pd, S->S2, S->S, S->R, S->health, list_check(S), s, S->mt, S->vw, S->rec,
+                                    S->subq);
+}
+
+/* Whether enqueue_integration launches anything, and how many kernels. */
+int integration_launches(const LqSim* S)
+{
+    const int sub = S->ph.constitutive_model == 3 ? 2 : 0;
+    return S->npm > 0 ? sub + (lqb::integrates_in_pair_kernel(S->pair_shape) ? 0 : 1) : 0;
 }
 
 /* The material slots' packed neighbour data after a filter changed S. */
@@ -414,9 +453,9 @@ int enqueue_rebuild(LqSim* S, cudaStream_t s)
                                                two_level(S) ? S->xwide : S->xbuild);
     LQ_TRY_CUDA(cudaGetLastError(), "k_copy_state");
     LQ_TRY(build_lists(S, s));
-    /* every slot's packed neighbour data (the boundary slots keep theirs
-     * until the next build) */
-    LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED));
+    /* every slot's packed neighbour data (the boundary slots keep theirs,
+     * in both stages' arrays, until the next build) */
+    LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, nullptr, S->rec2, S->npb));
     return lqb::launch_tile_order(ph, S->g.start, S->pair_shape, S->tile, s);
 }
 
@@ -453,29 +492,26 @@ int enqueue_density_filter(LqSim* S, cudaStream_t s)
  * writes the boundary slots' packed stress itself (boundary positions and
  * velocities are packed at each list build and do not change in between),
  * so the pair kernel needs no pack. */
-int enqueue_adami_pack(LqSim* S, const State& st, cudaStream_t s)
+int enqueue_adami_pack(LqSim* S, int stage, cudaStream_t s)
 {
-    /* both state buffers take the boundary stress, so their boundary slots
-     * stay equal and the integrators never touch them */
-    tensor2d* other = st.str == S->S.str ? S->S2.str : S->S.str;
-    return lqb::launch_adami_packed(&S->ph, S->pd, st, S->nlb, S->rec, s, other, S->bact, S->nbact);
+    /* both state buffers and both stages' records take the boundary
+     * stress, so their boundary slots stay equal and the integrators never
+     * touch them */
+    const bool first = stage == 1;
+    return lqb::launch_adami_packed(&S->ph, S->pd, first ? S->S : S->S2, S->nlb, first ? S->rec : S->rec2, s,
+                                    first ? S->S2.str : S->S.str, first ? S->rec2 : S->rec, S->bact, S->nbact);
 }
 
 
-/* The two stages of a step on the current lists. */
+/* The two stages of a step on the current lists: the predictor's (reference
+ * src/loquat.cu:343-368) and the corrector's (:371-396). */
 int enqueue_stages(LqSim* S, cudaStream_t s)
 {
-    const Parameters* ph = &S->ph;
-    const Parameters* pd = S->pd;
-    /* predictor stage (reference src/loquat.cu:343-368) */
-    LQ_TRY(enqueue_adami_pack(S, S->S, s));
-    LQ_TRY(enqueue_interaction(S, S->S, s));
-    LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true, S->subq));
-    /* corrector stage (reference src/loquat.cu:371-396) */
-    LQ_TRY(enqueue_adami_pack(S, S->S2, s));
-    LQ_TRY(enqueue_interaction(S, S->S2, s));
-    LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->R, S->health, list_check(S), s, S->mt, S->vw, S->rec,
-                                    S->subq));
+    for (int stage = 1; stage <= 2; ++stage) {
+        LQ_TRY(enqueue_adami_pack(S, stage, s));
+        LQ_TRY(enqueue_interaction(S, stage, s));
+        LQ_TRY(enqueue_integration(S, stage, s));
+    }
     return enqueue_dynamic_dt(S, s);
 }
 
@@ -695,6 +731,7 @@ int create(LqSim* S, const Parameters* par, const float* pos, const float* vel, 
         LQ_TRY(dev_alloc(S, (void**)&S->dtime, sizeof(double)));
     }
     LQ_TRY(dev_alloc(S, (void**)&S->rec, n * 13 * sizeof(float)));   /* cudaMalloc: 256-byte aligned */
+    LQ_TRY(dev_alloc(S, (void**)&S->rec2, n * 13 * sizeof(float)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.accad, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.spin, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.acestn, n * sizeof(tensor2d)));
@@ -1019,10 +1056,11 @@ extern "C" int lq_sim_launches_per_step(void* sim, int* plain, int* with_shepard
     if (!sim) return lqb::set_error(LQ_ERR_ARG, "lq_sim_launches_per_step: null sim");
     LqSim* S = static_cast<LqSim*>(sim);
     /* own kernels of a step without a rebuild: decide (graph only), Adami
-     * (when npb > 0), interaction and integrator (which packs the material
-     * slots' neighbour data) per stage; a Shepard pass adds the filter, its
-     * copy and the material pack */
-    const int stage = (S->npb > 0 ? 1 : 0) + 1 + 1;
+     * (when npb > 0) and the interaction per stage, which integrates its
+     * targets in the thread-per-target shapes, and what is left of the
+     * integration; a Shepard pass adds the filter, its copy and the
+     * material pack */
+    const int stage = (S->npb > 0 ? 1 : 0) + 1 + integration_launches(S);
     const int decide = S->conditional ? 1 : 0;
     const int dyn = (S->flags & LQ_SIM_DYNAMIC_DT) ? (S->npm > 0 ? 2 : 1) : 0;
     if (plain) *plain = decide + 2 * stage + dyn;
@@ -1572,7 +1610,7 @@ int profiled_step(LqSim* S, PhaseTimer& T)
         LQ_TRY(T.close(s));
         LQ_TRY(T.mark(s, PH_LIST));
         LQ_TRY(build_lists(S, s));
-        LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED));
+        LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, nullptr, S->rec2, S->npb));
         LQ_TRY(lqb::launch_tile_order(ph, S->g.start, S->pair_shape, S->tile, s));
         LQ_TRY(T.close(s));
     }
@@ -1581,22 +1619,18 @@ int profiled_step(LqSim* S, PhaseTimer& T)
         LQ_TRY(enqueue_renewal(S, s));
         LQ_TRY(T.close(s));
     }
-    State* cur[2] = {&S->S, &S->S2};
-    for (int stage = 0; stage < 2; ++stage) {
+    for (int stage = 1; stage <= 2; ++stage) {
         LQ_TRY(T.mark(s, PH_ADAMI));
-        LQ_TRY(enqueue_adami_pack(S, *cur[stage], s));
+        LQ_TRY(enqueue_adami_pack(S, stage, s));
         LQ_TRY(T.close(s));
         LQ_TRY(T.mark(s, PH_INTERACTION));
-        LQ_TRY(enqueue_interaction(S, *cur[stage], s));
+        LQ_TRY(enqueue_interaction(S, stage, s));
         LQ_TRY(T.close(s));
+        const bool dyn = stage == 2 && (S->flags & LQ_SIM_DYNAMIC_DT);
+        if (integration_launches(S) == 0 && !dyn) continue;
         LQ_TRY(T.mark(s, PH_INTEGRATE));
-        if (stage == 0)
-            LQ_TRY(lqb::launch_predict(ph, pd, S->S, S->S2, nullptr, S->R, s, S->mt, S->vw, S->rec, true, S->subq));
-        else {
-            LQ_TRY(lqb::launch_correct_into(ph, pd, S->S2, S->S, S->R, S->health, list_check(S), s, S->mt, S->vw,
-                                            S->rec, S->subq));
-            LQ_TRY(enqueue_dynamic_dt(S, s));
-        }
+        LQ_TRY(enqueue_integration(S, stage, s));
+        if (dyn) LQ_TRY(enqueue_dynamic_dt(S, s));
         LQ_TRY(T.close(s));
     }
     return LQ_OK;

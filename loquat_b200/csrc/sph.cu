@@ -26,6 +26,7 @@
 #include "lq_internal.cuh"
 #include "lq_tile.h"
 #include "lq_device.cuh"
+#include "lq_integrate.cuh"
 #include <adami_boundary.h>
 #include <field_smoothing.h>
 #include <particle_interaction.h>
@@ -294,17 +295,11 @@ __device__ __forceinline__ void pair_body_rec(const PairConst& K, const NbrArray
     }
 }
 
-/* The target's rates from its sums: acceleration and density rate, spin and
- * strain rate. */
-struct TargetRates {
-    float4 a, w;
-    tensor2d de;
-};
-
-__device__ __forceinline__ TargetRates rates_of(const Parameters* __restrict__ P, const PairConst& K, const Target& T)
+/* The target's rates from its sums. */
+__device__ __forceinline__ SlotRates rates_of(const Parameters* __restrict__ P, const PairConst& K, const Target& T)
 {
     const float c = K.mCg, hc = 0.5f * K.mCg;
-    TargetRates r;
+    SlotRates r;
     r.a = make_float4(fmaf(c, T.ax, __ldg(&P->acc_x)), fmaf(c, T.ay, __ldg(&P->acc_y)), fmaf(c, T.az, __ldg(&P->acc_z)),
                       c * T.drho);
     r.w = make_float4(hc * (T.l10 - T.l01), hc * (T.l20 - T.l02), hc * (T.l21 - T.l12), 0.0f);
@@ -316,7 +311,7 @@ __device__ __forceinline__ TargetRates rates_of(const Parameters* __restrict__ P
 __device__ __forceinline__ void store_rates(const Parameters* __restrict__ P, const PairConst& K, const Rates& rt,
                                             int i, const Target& T)
 {
-    const TargetRates r = rates_of(P, K, T);
+    const SlotRates r = rates_of(P, K, T);
     rt.accad[i] = r.a;
     rt.spin[i] = r.w;
     store_t2(rt.acestn, i, r.de);
@@ -493,10 +488,11 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
 }
 
 /* Slot i's packed record, at i or (with map) at map[i], the index lists
- * of another slot order gather it at (slots with none are skipped). */
+ * of another slot order gather it at (slots with none are skipped); the
+ * slots below n2 also into nb2. */
 template <bool kPk>
 __global__ void __launch_bounds__(kBlock) k_pack_neighbors(int first, int np, State st, NbrArrays nb,
-                                                           const int* __restrict__ map)
+                                                           const int* __restrict__ map, NbrArrays nb2, int n2)
 {
     const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
@@ -507,8 +503,9 @@ __global__ void __launch_bounds__(kBlock) k_pack_neighbors(int first, int np, St
     }
     const float4 x = __ldg(st.pos + i);
     const float4 v = __ldg(st.vel + i);
-    nb.xs[2 * (size_t)o] = make_float4(x.x, x.y, x.z, v.w);
-    store_packed<kPk>(nb, o, v, load_t2(st.str, i));
+    const tensor2d s = load_t2(st.str, i);
+    pack_slot<kPk>(nb, o, x, v, s);
+    if (i < n2) pack_slot<kPk>(nb2, o, x, v, s);
 }
 
 /* A list entry: each 128-byte row of a list is read once per launch, so it
@@ -701,17 +698,36 @@ __device__ __forceinline__ void list_sums(const PairConst& K, const NbrArrays& n
     }
 }
 
+/* What a stage's pair kernel does with a target's rates (StageOps): kStage 0
+ * stores them, 1 and 2 take the target's predictor or corrector step at
+ * once. */
+struct StageTail {
+    State in, out;          /* 1: state to stage buffer; 2: the snapshot, updated in place (out unused) */
+    MaterialTable mt;
+    NbrArrays nbw;          /* the records of the stage that follows */
+    int* health;
+    VerletCheck verlet;
+    bool keep_rates;        /* also store what later kernels of the stage read */
+};
+
 /* Pair sums over the lists from the packed neighbour arrays; a particle
  * whose list overflowed walks its stencil over the state arrays instead.
- * kThreads x kMinBlocks is the launch shape: the block size and
- * the resident blocks per SM the register allocation is capped for; the
- * shapes of kPairShapes are compiled and one is chosen per simulation
- * (lq_sim_autotune times them). */
-template <bool kKahan, int kThreads, int kMinBlocks>
+ * kThreads x kMinBlocks sets the register cap (kPairShapes).
+ *
+ * With kStage 1 or 2 the target is integrated where its sums end: the
+ * 56 bytes of rates are neither written nor read back, and the integrator's
+ * traffic, which as a kernel of its own runs at the memory's pace with the
+ * SMs' arithmetic idle, overlaps the other warps' pair sums: a step of
+ * the 1.97 M cylinder takes 1401 us so and 1501 with the integrators as
+ * kernels of their own (131 us each after pair launches of 605), the
+ * 5 k column 69 and 75.  The
+ * step writes the records that the next stage gathers, so the two stages'
+ * records are separate arrays: this one's are still being read. */
+template <bool kKahan, int kThreads, int kMinBlocks, int kStage>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
     const Parameters* __restrict__ P, int np, int npb, State st, Rates rt, Cells cells, const int* __restrict__ list,
     const int* __restrict__ count, int stride, Frames fr, NbrArrays nb, const int* __restrict__ order,
-    const int* __restrict__ rows)
+    const int* __restrict__ rows, StageTail tail)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= np - npb) return;
@@ -726,7 +742,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
      * index records packed in that other slot order, the target's own at
      * npb + row (the filler of the last group) */
     int row = t, self = i;
-    if (rows) {
+    if (kStage == 0 && rows) {
         row = __ldg(rows + t);
         self = npb + row;
     }
@@ -739,7 +755,22 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
     } else {
         walk_stencil(P, K, st, cells, i, T.x, [&](int j) { pair_body<kKahan>(K, st, T, j); }, fr);
     }
-    store_rates(P, K, rt, i, T);
+    if (kStage == 0) {
+        store_rates(P, K, rt, i, T);
+        return;
+    }
+    const SlotRates r = rates_of(P, K, T);
+    if (tail.keep_rates) {
+        rt.accad[i] = r.a;
+        rt.spin[i] = r.w;
+        store_t2(rt.acestn, i, r.de);
+    }
+    if (kStage == 1)
+        predict_slot<kKahan>(P, i, tail.in, tail.out, r, tail.mt, tail.nbw, true, tail.in.pos[i], tail.in.vel[i],
+                             tail.in.idep[i], load_t2_rw(tail.in.str, i), make_tensor2d(0.0f));
+    else
+        correct_slot<kKahan>(P, i, i, __ldg(&st.pos[i].w), tail.in.idep[i], tail.in, tail.in, r, tail.mt, tail.nbw,
+                             tail.health, tail.verlet);
 }
 
 /* ------------------------------------------------- tile order of targets */
@@ -1004,7 +1035,8 @@ template <int kG>
 __global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameters* __restrict__ P, int npb, State st,
                                                          const int* __restrict__ list,
                                                          const int* __restrict__ count, int stride, NbrArrays nb,
-                                                         tensor2d* __restrict__ str2, const int* __restrict__ act,
+                                                         NbrArrays nb2, tensor2d* __restrict__ str2,
+                                                         const int* __restrict__ act,
                                                          const int* __restrict__ nact)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1080,7 +1112,9 @@ __global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameter
         if (str2) store_t2(str2, i, out);
         /* a boundary particle's velocity and density stay as the list
          * build packed them; only its stress words change */
-        store_packed_stress(nb, i, __ldg(&st.vel[i].w), out);
+        const float rho = __ldg(&st.vel[i].w);
+        store_packed_stress(nb, i, rho, out);
+        if (nb2.xs) store_packed_stress(nb2, i, rho, out);
     }
 }
 
@@ -1400,32 +1434,34 @@ int launch_list_arrange(int n, const NeighborList& nl, cudaStream_t s)
 }
 
 int launch_pack_neighbors(const Parameters* ph, const State& st, float* rec, int first, cudaStream_t s,
-                          bool packed_velocity, const int* map)
+                          bool packed_velocity, const int* map, float* rec2, int n2)
 {
     const int n = ph->np - first;
     if (n <= 0) return LQ_OK;
     const NbrArrays nb = nbr_arrays(rec, ph->np);
+    const NbrArrays nb2 = rec2 ? nbr_arrays(rec2, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     if (packed_velocity)
-        k_pack_neighbors<true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map);
+        k_pack_neighbors<true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map, nb2, n2);
     else
-        k_pack_neighbors<false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map);
+        k_pack_neighbors<false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map, nb2, n2);
     LQ_TRY_CUDA(cudaGetLastError(), "k_pack_neighbors");
     return LQ_OK;
 }
 
 int launch_adami_packed(const Parameters* ph, const Parameters* pd, const State& st, const NeighborList& nl,
-                        float* rec, cudaStream_t s, tensor2d* str2, const int* act, const int* nact)
+                        float* rec, cudaStream_t s, tensor2d* str2, float* rec2, const int* act, const int* nact)
 {
     if (ph->npb <= 0) return LQ_OK;
     if (!act != !nact) return set_error(LQ_ERR_ARG, "Adami: compacted targets need both act and nact");
     if (nl.stride < ph->npb) return set_error(LQ_ERR_ARG, "Adami: list stride %d < %d targets", nl.stride, ph->npb);
     const NbrArrays nb = nbr_arrays(rec, ph->np);
+    const NbrArrays nb2 = rec2 ? nbr_arrays(rec2, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     const int grid = blocks_for(ph->npb, LQ_ADAMI_BLOCK);
     if (ph->npb >= kAdamiPairTargets)
-        k_adami_packed<2><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, str2, act,
+        k_adami_packed<2><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, nb2, str2, act,
                                                           nact);
     else
-        k_adami_packed<4><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, str2, act,
+        k_adami_packed<4><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, nb2, str2, act,
                                                           nact);
     LQ_TRY_CUDA(cudaGetLastError(), "k_adami_packed");
     return LQ_OK;
@@ -1475,66 +1511,85 @@ int launch_shepard_list(const Parameters* ph, const Parameters* pd, const State&
     return LQ_OK;
 }
 
+namespace {
+
+/* The pair kernel of a thread-per-target shape at stage kStage. */
+template <bool kKahan, int kStage>
+int launch_pair_stage(const Parameters* ph, const Parameters* pd, const State& st, const Rates& r, const Cells& c,
+                      const NeighborList& nl, cudaStream_t s, const Frames& fr, const NbrArrays& nb, int shape,
+                      const int* order, const int* rows, const StageTail& tail)
+{
+    const int threads = kPairShapes[shape][0], grid = blocks_for(ph->npm, threads);
+#define LQ_PAIR_LAUNCH(T, B)                                                                                          \
+    k_interaction_rec<kKahan, T, B, kStage><<<grid, threads, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, \
+                                                                     nl.stride, fr, nb, order, rows, tail)
+    /* one kernel per register cap, launched with each shape's block */
+    if constexpr (kStage == 0) {
+        LQ_PAIR_LAUNCH(768, 1);             /* 80 registers */
+    } else {
+        if (threads * kPairShapes[shape][1] == 768)
+            LQ_PAIR_LAUNCH(768, 1);         /* 80 */
+        else if (threads * kPairShapes[shape][1] == 640)
+            LQ_PAIR_LAUNCH(320, 2);         /* 96 */
+        else
+            LQ_PAIR_LAUNCH(128, 7);         /* 72 */
+    }
+#undef LQ_PAIR_LAUNCH
+    LQ_TRY_CUDA(cudaGetLastError(), "k_interaction_rec");
+    return LQ_OK;
+}
+
+}  // namespace
+
+bool integrates_in_pair_kernel(int shape) { return shape != 5 && shape != 6; }
+
 int launch_interaction_list(const Parameters* ph, const Parameters* pd, const State& st, const Rates& r,
                             const Cells& c, const NeighborList& nl, cudaStream_t s, const Frames& fr,
                             bool compensated, float* rec, int shape, bool pack, const int* order,
-                            const int* rows, const int* map)
+                            const int* rows, const int* map, const StageOps* ops)
 {
     if (ph->npm <= 0) return LQ_OK;
-    if (rec) {
-        if (reinterpret_cast<uintptr_t>(rec) % 32 != 0)
-            return set_error(LQ_ERR_ARG, "interaction: packed neighbour arrays must be 32-byte aligned");
-        const NbrArrays nb = nbr_arrays(rec, ph->np);
-        if (rows && (!map || !pack || shape == 5 || shape == 6))
-            return set_error(LQ_ERR_ARG, "interaction: list rows need a record map, a pack and a thread-per-target "
-                             "shape");
-        if (pack) LQ_TRY(launch_pack_neighbors(ph, st, rec, 0, s, compensated, rows ? map : nullptr));
-        if (shape >= 0 && shape < kPairShapeCount && kPairShapes[shape][2] == 1 && !order)
-            return set_error(LQ_ERR_ARG, "interaction: launch shape %d needs the tile order", shape);
-        if (shape < 0 || shape >= kPairShapeCount || kPairShapes[shape][2] != 1) order = nullptr;
-#define LQ_PAIR_LAUNCH(T, B)                                                                                \
-    (compensated ? k_interaction_rec<true, T, B><<<blocks_for(ph->npm, T), T, 0, s>>>(                      \
-                       pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, nl.stride, fr, nb, order, rows)       \
-                 : k_interaction_rec<false, T, B><<<blocks_for(ph->npm, T), T, 0, s>>>(                     \
-                       pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, nl.stride, fr, nb, order, rows))
-        switch (shape) {
-            case 7: LQ_PAIR_LAUNCH(768, 1); break;
-            case 8: LQ_PAIR_LAUNCH(384, 2); break;
-            case 9: LQ_PAIR_LAUNCH(256, 3); break;
-            case 10: LQ_PAIR_LAUNCH(320, 2); break;
-            case 1: LQ_PAIR_LAUNCH(64, 12); break;
-            case 2: LQ_PAIR_LAUNCH(256, 3); break;
-            case 3: LQ_PAIR_LAUNCH(128, 5); break;
-            case 4: LQ_PAIR_LAUNCH(128, 7); break;
-            case 5:
-            case 6: {
-                const int G = shape == 5 ? 8 : 32;
-                const int nthreads = ph->npm * G;
-                const int grid = (nthreads + 127) / 128;
-                if (G == 8) {
-                    if (compensated)
-                        k_interaction_group<true, 8><<<grid, 128, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list,
-                                                                          nl.count, nl.stride, fr, nb);
-                    else
-                        k_interaction_group<false, 8><<<grid, 128, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list,
-                                                                           nl.count, nl.stride, fr, nb);
-                } else {
-                    if (compensated)
-                        k_interaction_group<true, 32><<<grid, 128, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list,
-                                                                           nl.count, nl.stride, fr, nb);
-                    else
-                        k_interaction_group<false, 32><<<grid, 128, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list,
-                                                                            nl.count, nl.stride, fr, nb);
-                }
-                break;
-            }
-            default: LQ_PAIR_LAUNCH(kBlock, LQ_PAIR_MIN_BLOCKS); break;
+    if (!rec) return set_error(LQ_ERR_ARG, "interaction: the packed neighbour arrays are required");
+    if (reinterpret_cast<uintptr_t>(rec) % 32 != 0)
+        return set_error(LQ_ERR_ARG, "interaction: packed neighbour arrays must be 32-byte aligned");
+    if (shape < 0 || shape >= kPairShapeCount) return set_error(LQ_ERR_ARG, "interaction: launch shape %d", shape);
+    const NbrArrays nb = nbr_arrays(rec, ph->np);
+    if (rows && (!map || !pack || ops || shape == 5 || shape == 6))
+        return set_error(LQ_ERR_ARG, "interaction: list rows need a record map, a pack and a thread-per-target "
+                         "shape that stores its rates");
+    if (pack) LQ_TRY(launch_pack_neighbors(ph, st, rec, 0, s, compensated, rows ? map : nullptr));
+    if (kPairShapes[shape][2] == 1 && !order)
+        return set_error(LQ_ERR_ARG, "interaction: launch shape %d needs the tile order", shape);
+    if (kPairShapes[shape][2] != 1) order = nullptr;
+    if (shape == 5 || shape == 6) {
+        if (ops) return set_error(LQ_ERR_ARG, "interaction: launch shape %d stores its rates", shape);
+        const int G = shape == 5 ? 8 : 32;
+        const int grid = blocks_for((long long)ph->npm * G, 128);
+#define LQ_GROUP_LAUNCH(K, G)                                                                                   \
+    k_interaction_group<K, G><<<grid, 128, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, nl.stride, fr, nb)
+        if (G == 8) {
+            if (compensated) LQ_GROUP_LAUNCH(true, 8);
+            else LQ_GROUP_LAUNCH(false, 8);
+        } else {
+            if (compensated) LQ_GROUP_LAUNCH(true, 32);
+            else LQ_GROUP_LAUNCH(false, 32);
         }
-#undef LQ_PAIR_LAUNCH
-        LQ_TRY_CUDA(cudaGetLastError(), "k_interaction_rec");
+#undef LQ_GROUP_LAUNCH
+        LQ_TRY_CUDA(cudaGetLastError(), "k_interaction_group");
         return LQ_OK;
     }
-    return set_error(LQ_ERR_ARG, "interaction: the packed neighbour arrays are required");
+    if (!ops) {
+        if (compensated)
+            return set_error(LQ_ERR_ARG, "interaction: the compensated form integrates in the pair kernel");
+        return launch_pair_stage<false, 0>(ph, pd, st, r, c, nl, s, fr, nb, shape, order, rows, StageTail());
+    }
+    const StageTail tail{ops->in,     ops->out,   ops->mt, nbr_arrays(ops->rec_out, ph->np), ops->health,
+                         verlet_of(ph, ops->lists), ops->keep_rates || ph->constitutive_model == 3};
+    if (compensated)
+        return ops->stage == 1 ? launch_pair_stage<true, 1>(ph, pd, st, r, c, nl, s, fr, nb, shape, order, rows, tail)
+                               : launch_pair_stage<true, 2>(ph, pd, st, r, c, nl, s, fr, nb, shape, order, rows, tail);
+    return ops->stage == 1 ? launch_pair_stage<false, 1>(ph, pd, st, r, c, nl, s, fr, nb, shape, order, rows, tail)
+                           : launch_pair_stage<false, 2>(ph, pd, st, r, c, nl, s, fr, nb, shape, order, rows, tail);
 }
 
 int launch_adami(const Parameters* ph, const Parameters* pd, const State& st, const Cells& c, cudaStream_t s)
