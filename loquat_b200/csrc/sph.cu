@@ -118,8 +118,8 @@ __device__ __forceinline__ void load_target(const PairConst& K, const State& st,
         si = load_t2(st.str, i);
     }
     const float ri2 = 1.0f / (T.v.w * T.v.w);
-    T.Sxx = si.xx * ri2; T.Syy = si.yy * ri2; T.Szz = si.zz * ri2;
-    T.Sxy = si.xy * ri2; T.Sxz = si.xz * ri2; T.Syz = si.yz * ri2;
+    T.Sxx = __fmul_rn(si.xx, ri2); T.Syy = __fmul_rn(si.yy, ri2); T.Szz = __fmul_rn(si.zz, ri2);
+    T.Sxy = __fmul_rn(si.xy, ri2); T.Sxz = __fmul_rn(si.xz, ri2); T.Syz = __fmul_rn(si.yz, ri2);
     T.Rx = T.Ry = T.Rz = 0.f;
     if (K.artp) {
         T.Rx = si.xx > 0.f ? -K.eps * T.Sxx : 0.f;
@@ -295,16 +295,17 @@ __device__ __forceinline__ void pair_body_rec(const PairConst& K, const NbrArray
     }
 }
 
-/* The target's rates from its sums. */
+/* The target's rates from its sums; products rounded as such, whatever the
+ * kernel goes on to do with them. */
 __device__ __forceinline__ SlotRates rates_of(const Parameters* __restrict__ P, const PairConst& K, const Target& T)
 {
     const float c = K.mCg, hc = 0.5f * K.mCg;
     SlotRates r;
     r.a = make_float4(fmaf(c, T.ax, __ldg(&P->acc_x)), fmaf(c, T.ay, __ldg(&P->acc_y)), fmaf(c, T.az, __ldg(&P->acc_z)),
-                      c * T.drho);
-    r.w = make_float4(hc * (T.l10 - T.l01), hc * (T.l20 - T.l02), hc * (T.l21 - T.l12), 0.0f);
-    r.de = make_tensor2d(c * T.l00, c * T.l11, c * T.l22, hc * (T.l01 + T.l10), hc * (T.l02 + T.l20),
-                         hc * (T.l12 + T.l21));
+                      __fmul_rn(c, T.drho));
+    r.w = make_float4(__fmul_rn(hc, T.l10 - T.l01), __fmul_rn(hc, T.l20 - T.l02), __fmul_rn(hc, T.l21 - T.l12), 0.0f);
+    r.de = make_tensor2d(__fmul_rn(c, T.l00), __fmul_rn(c, T.l11), __fmul_rn(c, T.l22),
+                         __fmul_rn(hc, T.l01 + T.l10), __fmul_rn(hc, T.l02 + T.l20), __fmul_rn(hc, T.l12 + T.l21));
     return r;
 }
 
@@ -710,6 +711,25 @@ struct StageTail {
     bool keep_rates;        /* also store what later kernels of the stage read */
 };
 
+/* A target's step from its finished sums. */
+template <bool kKahan, int kStage>
+__device__ __forceinline__ void integrate_target(const Parameters* __restrict__ P, const PairConst& K, const Target& T,
+                                                 const State& st, const Rates& rt, int i, const StageTail& tail)
+{
+    const SlotRates r = rates_of(P, K, T);
+    if (tail.keep_rates) {
+        rt.accad[i] = r.a;
+        rt.spin[i] = r.w;
+        store_t2(rt.acestn, i, r.de);
+    }
+    if (kStage == 1)
+        predict_slot<kKahan>(P, i, tail.in, tail.out, r, tail.mt, tail.nbw, true, tail.in.pos[i], tail.in.vel[i],
+                             tail.in.idep[i], load_t2_rw(tail.in.str, i), make_tensor2d(0.0f));
+    else
+        correct_slot<kKahan>(P, i, i, __ldg(&st.pos[i].w), tail.in.idep[i], tail.in, tail.in, r, tail.mt, tail.nbw,
+                             tail.health, tail.verlet);
+}
+
 /* Pair sums over the lists from the packed neighbour arrays; a particle
  * whose list overflowed walks its stencil over the state arrays instead.
  * kThreads x kMinBlocks sets the register cap (kPairShapes).
@@ -759,18 +779,101 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
         store_rates(P, K, rt, i, T);
         return;
     }
-    const SlotRates r = rates_of(P, K, T);
-    if (tail.keep_rates) {
-        rt.accad[i] = r.a;
-        rt.spin[i] = r.w;
-        store_t2(rt.acestn, i, r.de);
+    integrate_target<kKahan, kStage>(P, K, T, st, rt, i, tail);
+}
+
+/* The pair kernel for few targets: a team of 16 lanes per target, with the
+ * sums of the thread-per-target form bit for bit.  A thread's list of about
+ * 80 entries is a chain of 20 groups of dependent gathers and about 8000
+ * instructions; below some 30 k targets there are too few warps to hide it
+ * and the launch takes 19 us whatever its size.  Here each lane forms the
+ * factors of one entry in 16 (the bulk of the work, in any order) and puts
+ * them into shared memory; then the lanes each own one of the target's 13
+ * sums and add the 16 terms in the list's order, in the groups of four of
+ * list_sums.  One warp of the block then integrates its targets.  A launch of
+ * 5 k targets takes 15 us instead of 23, one of 12 k 29 instead of 24: three
+ * times the work per target. */
+constexpr int kTeam = 16;
+constexpr int kTeamBlock = 128;
+template <bool kKahan, int kStage>
+__global__ void __launch_bounds__(kTeamBlock) k_interaction_team(
+    const Parameters* __restrict__ P, int np, int npb, State st, Rates rt, Cells cells, const int* __restrict__ list,
+    const int* __restrict__ count, int stride, Frames fr, NbrArrays nb, StageTail tail)
+{
+    __shared__ __align__(16) float val[kTeamBlock / kTeam][11][kTeam + 4];   /* rows on different banks */
+    __shared__ float sums[13][kTeamBlock / kTeam];
+    const int team = threadIdx.x / kTeam, c = threadIdx.x % kTeam;
+    const unsigned mates = 0xffffu << (threadIdx.x & 16);
+    const int first = npb + blockIdx.x * (kTeamBlock / kTeam);
+    const int i = first + team;
+    const PairConst K = load_pair_const(P);
+    Target T;
+    load_target(K, st, i < np ? i : first, true, T);
+    const int n = i < np ? __ldg(count + i - npb) : 0;
+    if (n <= LQ_NBR_CAP) {
+        /* the rows of val that lane c's sum multiplies: t3 and one of
+         * (vr, p), or one of -w and one of d; lanes 13 to 15 shadow 12 */
+        const int s = min(c, 12);
+        const int ra = s < 4 ? 0 : 5 + (s - 4) / 3, rb = s < 4 ? 1 + s : 8 + (s - 4) % 3;
+        const bool compensated = kKahan && s < 4;
+        const int n4 = (n + 3) & ~3;    /* the rows that the list's builder filled */
+        const int* p = list + (i - npb);
+        float sum = 0.0f, comp = 0.0f;
+        int j = c < n4 ? ld_list(p + (size_t)c * stride) : i;
+        for (int base = 0; base < n4; base += kTeam) {
+            PackedRecord<kKahan> r;
+            load_record(nb, lq_in_range(j, np) ? j : i, r);
+            const int k = base + kTeam + c;
+            j = k < n4 ? ld_list(p + (size_t)k * stride) : i;
+            const float3 vj = kKahan ? unpack_velocity(r.sb.z, r.sb.w) : make_float3(r.sb.z, r.sb.w, r.vz);
+            const tensor2d sj = make_tensor2d(r.sa.x, r.sa.y, r.sa.z, r.sa.w, r.sb.x, r.sb.y);
+            const PairFactors f = K.artp ? pair_factors<true>(K, T, r.xr, vj, sj) : pair_factors<false>(K, T, r.xr, vj, sj);
+            float(&v)[11][kTeam + 4] = val[team];
+            v[0][c] = f.t3;
+            v[1][c] = f.vr;
+            v[2][c] = f.px;
+            v[3][c] = f.py;
+            v[4][c] = f.pz;
+            v[5][c] = -f.wx;
+            v[6][c] = -f.wy;
+            v[7][c] = -f.wz;
+            v[8][c] = f.dx;
+            v[9][c] = f.dy;
+            v[10][c] = f.dz;
+            __syncwarp(mates);
+#pragma unroll
+            for (int m = 0; m < kTeam / 4; ++m)
+                if (base + 4 * m < n4) {
+                    const float4 a = *reinterpret_cast<const float4*>(&v[ra][4 * m]);
+                    const float4 b = *reinterpret_cast<const float4*>(&v[rb][4 * m]);
+                    float d = compensated ? 0.0f : sum;
+                    d = fmaf(a.x, b.x, d);
+                    d = fmaf(a.y, b.y, d);
+                    d = fmaf(a.z, b.z, d);
+                    d = fmaf(a.w, b.w, d);
+                    if (compensated)
+                        kahan_add(sum, comp, d);
+                    else
+                        sum = d;
+                }
+            __syncwarp(mates);
+        }
+        if (c < 13) sums[c][team] = sum;
+    } else if (c == 0) {
+        walk_stencil(P, K, st, cells, i, T.x, [&](int j) { pair_body<kKahan>(K, st, T, j); }, fr);
+        const float of[13] = {T.drho, T.ax, T.ay, T.az, T.l00, T.l01, T.l02, T.l10, T.l11, T.l12, T.l20, T.l21, T.l22};
+#pragma unroll
+        for (int k = 0; k < 13; ++k) sums[k][team] = of[k];
     }
-    if (kStage == 1)
-        predict_slot<kKahan>(P, i, tail.in, tail.out, r, tail.mt, tail.nbw, true, tail.in.pos[i], tail.in.vel[i],
-                             tail.in.idep[i], load_t2_rw(tail.in.str, i), make_tensor2d(0.0f));
-    else
-        correct_slot<kKahan>(P, i, i, __ldg(&st.pos[i].w), tail.in.idep[i], tail.in, tail.in, r, tail.mt, tail.nbw,
-                             tail.health, tail.verlet);
+    __syncthreads();
+    const int x = threadIdx.x;
+    if (x >= kTeamBlock / kTeam || first + x >= np) return;
+    T.drho = sums[0][x];
+    T.ax = sums[1][x]; T.ay = sums[2][x]; T.az = sums[3][x];
+    T.l00 = sums[4][x]; T.l01 = sums[5][x]; T.l02 = sums[6][x];
+    T.l10 = sums[7][x]; T.l11 = sums[8][x]; T.l12 = sums[9][x];
+    T.l20 = sums[10][x]; T.l21 = sums[11][x]; T.l22 = sums[12][x];
+    integrate_target<kKahan, kStage>(P, K, T, st, rt, first + x, tail);
 }
 
 /* ------------------------------------------------- tile order of targets */
@@ -994,6 +1097,30 @@ __global__ void __launch_bounds__(kBlock) k_shepard(const Parameters* __restrict
     }
 }
 
+/* A boundary particle's stress from the sums of its extrapolation (sigma_j
+ * V_j W in S, x_ij V_j W and V_j W in acc), into both state buffers and both
+ * stages' records; a boundary particle's velocity and density stay as the
+ * list build packed them, only its stress words change. */
+__device__ __forceinline__ void store_wall_stress(const Parameters* __restrict__ P, const State& st, int i,
+                                                  const tensor2d& S, const float4& acc, tensor2d* str2,
+                                                  const NbrArrays& nb, const NbrArrays& nb2)
+{
+    const float rho0 = __ldg(&P->rho0);
+    const float inv = 1.0f / acc.w;
+    tensor2d out;
+    out.xx = (S.xx - rho0 * __ldg(&P->acc_x) * acc.x) * inv;
+    out.yy = (S.yy - rho0 * __ldg(&P->acc_y) * acc.y) * inv;
+    out.zz = (S.zz - rho0 * __ldg(&P->acc_z) * acc.z) * inv;
+    out.xy = S.xy * inv;
+    out.xz = S.xz * inv;
+    out.yz = S.yz * inv;
+    store_t2(st.str, i, out);
+    if (str2) store_t2(str2, i, out);
+    const float rho = __ldg(&st.vel[i].w);
+    store_packed_stress(nb, i, rho, out);
+    if (nb2.xs) store_packed_stress(nb2, i, rho, out);
+}
+
 /* ------------------------------------------------- list-driven Adami */
 /* The Adami extrapolation of k_adami, summed over a boundary particle's
  * list of material neighbours (built with a skin; pairs at q >= 2 add
@@ -1031,6 +1158,14 @@ __global__ void __launch_bounds__(kBlock) k_shepard(const Parameters* __restrict
 #define LQ_ADAMI_PAIR_TARGETS (4 << 20)
 #endif
 constexpr int kAdamiPairTargets = LQ_ADAMI_PAIR_TARGETS;
+/* Boundary particles below which each compacted target gets eight lanes
+: below it the gathers' latency is the time (345 k:
+ * 24 us a launch with one lane, 20 with eight), above it their number
+ * (1.9 M: 90 us with one lane each; not measured with eight). */
+#ifndef LQ_ADAMI_GROUP_TARGETS
+#define LQ_ADAMI_GROUP_TARGETS (1 << 20)
+#endif
+constexpr int kAdamiGroupTargets = LQ_ADAMI_GROUP_TARGETS;
 template <int kG>
 __global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameters* __restrict__ P, int npb, State st,
                                                          const int* __restrict__ list,
@@ -1098,23 +1233,76 @@ __global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameter
             acc.w += kv;
         }
     }
-    if (acc.w > 0.0f) {
-        const float rho0 = __ldg(&P->rho0);
-        const float inv = 1.0f / acc.w;
-        tensor2d out;
-        out.xx = (S.xx - rho0 * __ldg(&P->acc_x) * acc.x) * inv;
-        out.yy = (S.yy - rho0 * __ldg(&P->acc_y) * acc.y) * inv;
-        out.zz = (S.zz - rho0 * __ldg(&P->acc_z) * acc.z) * inv;
-        out.xy = S.xy * inv;
-        out.xz = S.xz * inv;
-        out.yz = S.yz * inv;
-        store_t2(st.str, i, out);
-        if (str2) store_t2(str2, i, out);
-        /* a boundary particle's velocity and density stay as the list
-         * build packed them; only its stress words change */
-        const float rho = __ldg(&st.vel[i].w);
-        store_packed_stress(nb, i, rho, out);
-        if (nb2.xs) store_packed_stress(nb2, i, rho, out);
+    if (acc.w > 0.0f) store_wall_stress(P, st, i, S, acc, str2, nb, nb2);
+}
+
+/* The list-driven Adami with G lanes per target, for the sizes at which
+ * k_adami_packed's chain of dependent gathers is the time (16 us a launch
+ * from 5 k to 1 M particles; 9.5 so, 17 at the 1.97 M cylinder): lane g
+ * takes entries g, g + G, ..., two at a time, and the ten sums are combined
+ * with shuffles.  A fixed grid walks the compacted targets, whose number
+ * only the device knows. */
+template <int G>
+__global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_group(const Parameters* __restrict__ P, State st,
+                                                                const int* __restrict__ list,
+                                                                const int* __restrict__ count, int stride,
+                                                                NbrArrays nb, NbrArrays nb2,
+                                                                tensor2d* __restrict__ str2,
+                                                                const int* __restrict__ act,
+                                                                const int* __restrict__ nact)
+{
+    const int g = threadIdx.x % G;
+    const unsigned mates = (unsigned)((1ull << G) - 1ull) << (threadIdx.x & 31 & ~(G - 1));
+    const int step = gridDim.x * (LQ_ADAMI_BLOCK / G), na = __ldg(nact);
+    const int np_all = __ldg(&P->np);
+    const float ih = __ldg(&P->i_h), m = __ldg(&P->m), Cw = __ldg(&P->kernel_normalization_par);
+    for (int a = (blockIdx.x * LQ_ADAMI_BLOCK + threadIdx.x) / G; a < na; a += step) {
+        const int i = __ldg(act + a);
+        const int n = min(__ldg(count + i), LQ_NBR_CAP);
+        const float4 xi = __ldg(st.pos + i);
+        float sum[10] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const int* p = list + i;
+        for (int k = g; k < n; k += 2 * G) {
+            int j[2];
+            float4 xr[2], sa[2];
+            float2 sb[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                j[u] = k + u * G < n ? __ldg(p + (size_t)(k + u * G) * stride) : i;
+                if (!lq_in_range(j[u], np_all)) j[u] = i;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                load_xs(nb, j[u], xr[u], sa[u]);
+                sb[u] = __ldg(reinterpret_cast<const float2*>(nb.sb + j[u]));
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float dx = xi.x - xr[u].x, dy = xi.y - xr[u].y, dz = xi.z - xr[u].z;
+                const float q = sqrt_approx(dx * dx + dy * dy + dz * dz) * ih;
+                const float t = k + u * G < n ? fmaxf(2.0f - q, 0.0f) : 0.0f;
+                const float ker = Cw * t * t * t * t * (q + 0.5f);
+                const float kv = ker * __fdividef(m, xr[u].w);
+                const float cs = m * xr[u].w * ker;
+                sum[0] += sa[u].x * cs;
+                sum[1] += sa[u].y * cs;
+                sum[2] += sa[u].z * cs;
+                sum[3] += sa[u].w * cs;
+                sum[4] += sb[u].x * cs;
+                sum[5] += sb[u].y * cs;
+                sum[6] += dx * kv;
+                sum[7] += dy * kv;
+                sum[8] += dz * kv;
+                sum[9] += kv;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 10; ++k)
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(mates, sum[k], o, G);
+        if (g == 0 && sum[9] > 0.0f)
+            store_wall_stress(P, st, i, make_tensor2d(sum[0], sum[1], sum[2], sum[3], sum[4], sum[5]),
+                              make_float4(sum[6], sum[7], sum[8], sum[9]), str2, nb, nb2);
     }
 }
 
@@ -1457,7 +1645,14 @@ int launch_adami_packed(const Parameters* ph, const Parameters* pd, const State&
     const NbrArrays nb = nbr_arrays(rec, ph->np);
     const NbrArrays nb2 = rec2 ? nbr_arrays(rec2, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     const int grid = blocks_for(ph->npb, LQ_ADAMI_BLOCK);
-    if (ph->npb >= kAdamiPairTargets)
+    if (act && ph->npb < kAdamiGroupTargets) {
+        int dev = 0, sms = 0;
+        LQ_TRY_CUDA(cudaGetDevice(&dev), "Adami");
+        LQ_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "Adami");
+        const int all = blocks_for((long long)ph->npb * 8, LQ_ADAMI_BLOCK), most = sms * 12;
+        k_adami_group<8><<<all < most ? all : most, LQ_ADAMI_BLOCK, 0, s>>>(pd, st, nl.list, nl.count, nl.stride, nb,
+                                                                            nb2, str2, act, nact);
+    } else if (ph->npb >= kAdamiPairTargets)
         k_adami_packed<2><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, nb2, str2, act,
                                                           nact);
     else
@@ -1513,12 +1708,26 @@ int launch_shepard_list(const Parameters* ph, const Parameters* pd, const State&
 
 namespace {
 
+/* Shape 0 gives each target a team of lanes up to this many: between the
+ * 5 k and 12 k at which the two forms were measured (k_interaction_team). */
+#ifndef LQ_TEAM_TARGETS
+#define LQ_TEAM_TARGETS 8192
+#endif
+constexpr int kTeamTargets = LQ_TEAM_TARGETS;
+
 /* The pair kernel of a thread-per-target shape at stage kStage. */
 template <bool kKahan, int kStage>
 int launch_pair_stage(const Parameters* ph, const Parameters* pd, const State& st, const Rates& r, const Cells& c,
                       const NeighborList& nl, cudaStream_t s, const Frames& fr, const NbrArrays& nb, int shape,
                       const int* order, const int* rows, const StageTail& tail)
 {
+    if constexpr (kStage != 0)
+        if (shape == 0 && ph->npm <= kTeamTargets) {
+            k_interaction_team<kKahan, kStage><<<blocks_for(ph->npm, kTeamBlock / kTeam), kTeamBlock, 0, s>>>(
+                pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, nl.stride, fr, nb, tail);
+            LQ_TRY_CUDA(cudaGetLastError(), "k_interaction_team");
+            return LQ_OK;
+        }
     const int threads = kPairShapes[shape][0], grid = blocks_for(ph->npm, threads);
 #define LQ_PAIR_LAUNCH(T, B)                                                                                          \
     k_interaction_rec<kKahan, T, B, kStage><<<grid, threads, 0, s>>>(pd, ph->np, ph->npb, st, r, c, nl.list, nl.count, \
