@@ -355,27 +355,37 @@ __device__ __forceinline__ void walk_stencil(const Parameters* __restrict__ P, c
 #endif
 
 constexpr int kListWarps = kBlock / 32;
-constexpr int kStage = 32;
-constexpr int kUnroll = 8;
+constexpr int kListChunk = 128;     /* candidates a warp holds at once, four a lane */
 
 /* Neighbour lists: list[k * stride + t] is the k-th neighbour slot of target
  * slot first + t, count[t] their number (entries past LQ_NBR_CAP are not
  * stored).  Candidates come from grid layers layer_lo..1 (0: both layers,
  * 1: material only) and are kept when r^2 < cut2, the cut-off (2h) plus any
- * skin.  Lanes are grouped by grid column; each group
- * walks the union of its lanes' stencils, so the loop and every candidate
- * load are warp-uniform and each lane only runs its distance test.  A lane's
- * own slot passes the test too: its pair adds exactly zero.  Along z the
- * walk covers every cell the lane's cut-off sphere reaches (two cells down
- * or up when the particle lies within the skin of a cell face), so a list
- * holds all its particle's pairs within the cut-off in those columns,
- * whatever the group; across columns it covers the 3 x 3 around the
- * particle's own, which holds every pair within 2h.  A pair within
- * 2h + skin that lies two columns apart is left out: it is more than 2h
- * apart when the list is built, so until the next build its distance stays
- * above 2h - skin (q > 2 - skin/h), where the kernel factor (2 - q)^3 stays
- * below (skin/h)^3.  Hits are staged per lane in shared memory and flushed
- * in rows.
+ * skin, in the order of the walk: layer, column (dy outer, dx inner), slot.
+ * A lane's own slot passes the test too: its pair adds exactly zero.  Along
+ * z the walk covers every cell the target's cut-off sphere reaches (two
+ * cells down or up when the particle lies within the skin of a cell face),
+ * so a list holds all its particle's pairs within the cut-off in those
+ * columns; across columns it covers the 3 x 3 around the particle's own,
+ * which holds every pair within 2h.  A pair within 2h + skin that lies two
+ * columns apart is left out: it is more than 2h apart when the list is
+ * built, so until the next build its distance stays above 2h - skin
+ * (q > 2 - skin/h), where the kernel factor (2 - q)^3 stays below
+ * (skin/h)^3.
+ *
+ * A warp's targets are grouped by grid column; for each group the warp
+ * walks the union of their stencils, one contiguous slot range per column
+ * and layer, joined to one sequence of about 700 candidates.  The lanes
+ * hold 128 of them at once from coalesced loads and test them against one
+ * target after the other (broadcast from shared memory, each coordinate
+ * twice, for the paired FP32 instructions that take two candidates); votes
+ * give the target's hits as bit masks, from which its own lane then writes
+ * its list.  Bound by issue slots.  With a lane per target and a broadcast
+ * load per candidate, each candidate took four passes of the L1 data pipe
+ * to reach the lanes (79 % busy) and eight instructions a lane instead of
+ * six.  At 786 k
+ * targets 377 us against 496, and in small cases, where the loads' latency
+ * was the time, 107 us for all lists of the 5 k column against 204.
  *
  * With `shell` (the wide build of two-level lists) the hits are split: those
  * with r^2 < inner2 go to `list` (count_out[t] of them) and the rest to
@@ -392,45 +402,22 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
                                                           const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;     /* the whole grid leaves: no collective is split */
-    __shared__ int stage[kListWarps][kStage][32];
+    __shared__ float4 target_xy[kListWarps][32];    /* x, x, y, y */
+    __shared__ float2 target_z[kListWarps][32];     /* z, z */
+    __shared__ int slot[kListWarps][kListChunk];
+    __shared__ uint4 hits[kListWarps][32], ins[kListWarps][kSplit ? 32 : 1];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = first + t;
     const bool active = t < ntarget;
-    const PairConst K = load_pair_const(P);
+    const float ih = __ldg(&P->i_h);
     const int nx = __ldg(&P->cell_num_x), ny = __ldg(&P->cell_num_y), nz = __ldg(&P->cell_num_z);
     const int L = __ldg(&P->ncell_one_layer);
     const int np_all = __ldg(&P->np);
     const float4 xi = active ? __ldg(pos + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    int* my_stage = &stage[w][0][lane];
-
-    /* staged hits carry bit 31 when they go to the shell part */
-    int staged = 0, ni = 0, ns = 0;
-    auto flush = [&]() {
-        const int maxc = (int)__reduce_max_sync(FULL, (unsigned)staged);
-        for (int k = 0; k < maxc; ++k)
-            if (k < staged) {
-                const int e = my_stage[32 * k];
-                if (kSplit && e < 0) {
-                    if (ns < LQ_NBR_CAP) shell[(size_t)ns * stride + t] = e & 0x7fffffff;
-                    ++ns;
-                } else {
-                    if (ni < LQ_NBR_CAP) list[(size_t)ni * stride + t] = e;
-                    ++ni;
-                }
-            }
-        staged = 0;
-        __syncwarp();
-    };
-    auto test = [&](bool mine, const float4& xj, int j) {
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (mine && r2 < cut2) {
-            my_stage[32 * staged] = (kSplit && !(r2 < inner2)) ? (int)((unsigned)j | 0x80000000u) : j;
-            ++staged;
-        }
-    };
+    target_xy[w][lane] = make_float4(xi.x, xi.x, xi.y, xi.y);
+    target_z[w][lane] = make_float2(xi.z, xi.z);
 
     /* the z cells the particle's cut-off sphere reaches (a run walks the
      * group's union of them), so a lane's list never depends on which
@@ -438,45 +425,130 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
     const float cut = sqrtf(cut2);
     int cx = 0, cy = 0, czl = 0, czh = 0;
     if (active) {
-        cx = stencil_axis(xi.x, K.ih);
-        cy = stencil_axis(xi.y, K.ih);
-        czl = stencil_axis(xi.z - cut, K.ih);
-        czh = stencil_axis(xi.z + cut, K.ih);
+        cx = stencil_axis(xi.x, ih);
+        cy = stencil_axis(xi.y, ih);
+        czl = stencil_axis(xi.z - cut, ih);
+        czh = stencil_axis(xi.z + cut, ih);
         if (fr.rows) cy = frame_stencil_row(fr, __ldg(&idep[i].x), cy);
     }
+    int ni = 0, ns = 0;
     unsigned todo = __ballot_sync(FULL, active);
+    __syncwarp();
     while (todo) {
         const int leader = __ffs(todo) - 1;
         const int gx = __shfl_sync(FULL, cx, leader), gy = __shfl_sync(FULL, cy, leader);
         const bool mine = active && cx == gx && cy == gy;
-        todo &= ~__ballot_sync(FULL, mine);
+        const unsigned group = __ballot_sync(FULL, mine);
+        const int lo = __ffs(group) - 1, hi = 31 - __clz(group);
+        todo &= ~group;
         const int zmin = __reduce_min_sync(FULL, mine ? czl : INT_MAX);
         const int zmax = __reduce_max_sync(FULL, mine ? czh : INT_MIN);
         const int zlo = max(zmin, 0), zhi = min(zmax, nz - 1);
         if (zlo > zhi) continue;
-        for (int layer = layer_lo; layer < 2; ++layer) {
-            const int off = layer ? L : 0;
-            for (int col = 0; col < 9; ++col) {
-                const int X = gx + (col % 3) - 1, Y = gy + (col / 3) - 1;
-                if (X < 0 || X >= nx || Y < 0 || Y >= ny) continue;
-                int s, e;
-                if (!zrun_range(cells, off + (X * ny + Y) * nz, zlo, zhi, s, e)) continue;
-                if (!lq_in_range(s, np_all) || !lq_in_range(e - 1, np_all)) continue;
-                int j = s;
-                for (; j + kUnroll <= e; j += kUnroll) {
-                    if (__any_sync(FULL, staged > kStage - kUnroll)) flush();
-                    float4 xj[kUnroll];
+        /* lane r < 9 per layer: the slot range [s, s + len) of run r, which
+         * begins at place `at` of the joined sequence */
+        int s = 0, len = 0;
+        {
+            const int layer = layer_lo + lane / 9, col = lane % 9;
+            const int X = gx + (col % 3) - 1, Y = gy + (col / 3) - 1;
+            int e;
+            if (layer < 2 && X >= 0 && X < nx && Y >= 0 && Y < ny &&
+                zrun_range(cells, (layer ? L : 0) + (X * ny + Y) * nz, zlo, zhi, s, e) && lq_in_range(s, np_all) &&
+                lq_in_range(e - 1, np_all))
+                len = e - s;
+        }
+        int end = len;
 #pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) xj[u] = __ldg(pos + j + u);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, end, o);
+            if (lane >= o) end += v;
+        }
+        const int at = end - len, total = __shfl_sync(FULL, end, 31);
+        unsigned runs = __ballot_sync(FULL, len > 0);       /* from the one that holds `base` on */
+        for (int base = 0; base < total; base += kListChunk) {
+            /* lane l holds places base + 32 c + l: their slots and, negated,
+             * their positions, far beyond any cut-off past the end */
+            int j[4] = {-1, -1, -1, -1};
+            int last = 0;
+            for (unsigned m = runs; m; m &= m - 1) {
+                const int r = __ffs(m) - 1;
+                const int ra = __shfl_sync(FULL, at, r), rs = __shfl_sync(FULL, s, r);
+                if (ra >= base + kListChunk) break;
+                last = r;
 #pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) test(mine, xj[u], j + u);
+                for (int c = 0; c < 4; ++c) {
+                    const int q = base + 32 * c + lane;
+                    if (q >= ra && q < total) j[c] = rs + (q - ra);
                 }
-                if (__any_sync(FULL, staged > kStage - kUnroll)) flush();
-                for (; j < e; ++j) test(mine, __ldg(pos + j), j);
             }
+            runs &= ~0u << last;
+            float4 x[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                x[c] = j[c] >= 0 ? __ldg(pos + j[c]) : make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f);
+                slot[w][32 * c + lane] = j[c];
+            }
+            float2 mx[2], my[2], mz[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                mx[c] = make_float2(-x[2 * c].x, -x[2 * c + 1].x);
+                my[c] = make_float2(-x[2 * c].y, -x[2 * c + 1].y);
+                mz[c] = make_float2(-x[2 * c].z, -x[2 * c + 1].z);
+            }
+            /* the group's lanes are neighbours (slots of one column follow
+             * one another); a lane between them that is not of the group
+             * leaves its masks unread */
+#pragma unroll 2
+            for (int tt = lo; tt <= hi; ++tt) {
+                const float4 xy = target_xy[w][tt];
+                const float2 tx = make_float2(xy.x, xy.y), ty = make_float2(xy.z, xy.w), tz = target_z[w][tt];
+                unsigned h[4], b[4];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float2 dx = __fadd2_rn(tx, mx[c]), dy = __fadd2_rn(ty, my[c]), dz = __fadd2_rn(tz, mz[c]);
+                    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                    h[2 * c] = __ballot_sync(FULL, r2.x < cut2);
+                    h[2 * c + 1] = __ballot_sync(FULL, r2.y < cut2);
+                    if (kSplit) {
+                        b[2 * c] = __ballot_sync(FULL, r2.x < inner2);
+                        b[2 * c + 1] = __ballot_sync(FULL, r2.y < inner2);
+                    }
+                }
+                if (lane == 0) {
+                    hits[w][tt] = make_uint4(h[0], h[1], h[2], h[3]);
+                    if (kSplit) ins[w][tt] = make_uint4(b[0], b[1], b[2], b[3]);
+                }
+            }
+            /* each lane's hits, in the sequence's order */
+            __syncwarp();
+            const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+            const uint4 h4 = mine ? hits[w][lane] : none, b4 = mine && kSplit ? ins[w][kSplit ? lane : 0] : none;
+            const unsigned hit[4] = {h4.x, h4.y, h4.z, h4.w}, in[4] = {b4.x, b4.y, b4.z, b4.w};
+            int c = 0;
+            unsigned h = hit[0], b = in[0];
+            for (;;) {
+#pragma unroll
+                for (int k = 1; k < 4; ++k)
+                    if (h == 0 && c < k) {
+                        c = k;
+                        h = hit[k];
+                        b = in[k];
+                    }
+                if (h == 0) break;
+                const int bit = __ffs(h) - 1;
+                h &= h - 1;
+                const int hj = slot[w][32 * c + bit];
+                if (kSplit && !(b >> bit & 1u)) {
+                    if (ns < LQ_NBR_CAP) shell[(size_t)ns * stride + t] = hj;
+                    ++ns;
+                } else {
+                    if (ni < LQ_NBR_CAP) list[(size_t)ni * stride + t] = hj;
+                    ++ni;
+                }
+            }
+            __syncwarp();
         }
     }
-    flush();
     if (active) {
         /* the list's last group of four filled up with the target itself
          * (the split build's lists are filled up by their renewal) */
