@@ -187,8 +187,6 @@ struct StageOps {
 };
 
 /* ------------------------------------------------------------ operators */
-int launch_neighbor_list(const Parameters* par_host, const Parameters* par_dev, const float4* pos, const Cells& c,
-                         const NeighborList& nl, cudaStream_t s);
 /* `rec` (np x 13 floats, 32-byte aligned; required) holds the neighbour
  * data packed into dense arrays (position and density, velocity and
  * sigma/rho^2: 52 bytes per particle, 48 in the compensated form, whose
@@ -255,11 +253,9 @@ int tile_order_scratch(const Parameters* par_host, int* nseg, size_t* scan_bytes
 int launch_tile_order(const Parameters* par_host, const int* start, int shape, const TileOrder& to, cudaStream_t s);
 int launch_adami(const Parameters* par_host, const Parameters* par_dev, const State& st, const Cells& c,
                  cudaStream_t s);
-/* Shepard filter of material stress into out_str[npb, np).  When `full` is
- * set the kernel also copies every other array (and the boundary stress)
- * from `st` to `out`, producing a complete new state. */
+/* Shepard filter of material stress into out_str[npb, np). */
 int launch_shepard(const Parameters* par_host, const Parameters* par_dev, const State& st, tensor2d* out_str,
-                   const State* full, const Cells& c, cudaStream_t s);
+                   const Cells& c, cudaStream_t s);
 /* Predictor: out <- in advanced by dt/2 on material slots; boundary slots
  * are left alone (the native driver's Adami writes both of its state
  * buffers), except that with a snapshot `snap` (may be all-null), which

@@ -12,7 +12,7 @@ from loquat_b200 import cases
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("size,hdr", [((1, 1, 1), 1.2), ((5, 3, 2), 1.2), ((2, 9, 31), 1.3), ((40, 3, 3), 1.0),
+@pytest.mark.parametrize("size,hdr", [((1, 1, 5), 1.2), ((5, 3, 2), 1.2), ((2, 9, 31), 1.3), ((40, 3, 3), 1.0),
                                       ((12, 11, 13), 1.5)])
 @pytest.mark.parametrize("skin", [0.0, 0.05])
 def test_list_entries_are_the_pairs_within_the_cut_off(lq, cuda, size, hdr, skin):
@@ -39,6 +39,7 @@ def test_list_entries_are_the_pairs_within_the_cut_off(lq, cuda, size, hdr, skin
         i, j = np.array(i, int), np.array(j, int)
         return int(np.sum(np.all(np.abs(col[i] - col[j]) <= 1, axis=1)))
 
+    assert not s.health().any()     # every particle lies in the lattice
     soil, wall, every = np.arange(nb, c.par.np), np.arange(nb), np.arange(c.par.np)
     cut = (2.0 + skin) * h
     for got, targets, sources in ((material, soil, every), (boundary, wall, soil)):
