@@ -10,15 +10,16 @@
  *   3. k_scatter     slot = start[key] + rank
  *   4. k_cell_order  ranks from atomics are not ordered across warps, so each
  *                    cell's slot range is put back in ascending previous-slot
- *                    order (insertion sort; input order is nearly sorted
- *                    because particles move little between searches).  The
- *                    result equals a stable sort by key, bit for bit.
- *   5. k_bounds      per-cell begin/end (-1 when empty), only for callers of
- *                    the reference interface; the native driver reads the
- *                    start table directly.
+ *                    order; the result equals a stable sort by key, bit for
+ *                    bit.  The same pass writes what follows from the order:
+ *                    the sorted keys, the per-cell begin/end (-1 when empty)
+ *                    for callers of the reference interface (the native
+ *                    driver reads the start table directly) and the slots'
+ *                    particle identities.
  * HBM traffic per particle: 16 B position read, 8 B key+rank written and read
  * back, 8 B sorted outputs; plus 12 B per cell for count, start and bounds.
  */
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -88,48 +89,112 @@ __global__ void __launch_bounds__(kBlock) k_fill_int(int* __restrict__ p, int n,
 __global__ void k_add_int(int* __restrict__ p, int v) { *p += v; }
 
 __global__ void __launch_bounds__(kBlock) k_scatter(int np, const int* __restrict__ key, const int* __restrict__ rank,
-                                                    const int* __restrict__ start, int* __restrict__ part_idx,
-                                                    int* __restrict__ part_cel)
+                                                    const int* __restrict__ start, int* __restrict__ part_idx)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    const int k = key[i];
-    const int d = __ldg(start + k) + rank[i];
-    if (!lq_in_range(d, np)) return;
-    part_idx[d] = i;
-    part_cel[d] = k;
+    const int d = __ldg(start + key[i]) + rank[i];
+    if (lq_in_range(d, np)) part_idx[d] = i;
 }
 
-__global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, const int* __restrict__ start,
-                                                       int* __restrict__ part_idx)
+/* What a search writes of its order besides part_idx: the sorted keys, the
+ * per-cell bounds and the identities of the slots' particles (each may be
+ * null; ident_out[slot] = ident_in[previous slot]). */
+struct OrderOutputs {
+    int* part_cel;
+    int* beg;
+    int* end;
+    const int* ident_in;
+    int* ident_out;
+};
+
+/* A warp takes 32 cells, one after the other: the lanes load a cell's slots
+ * (the next cell's meanwhile), a vote tells whether they are in order, and
+ * if not each lane finds its particle's place by counting the smaller ones.
+ * One thread per cell, inserting, was a chain of about 17 dependent loads
+ * and stores with most threads of a warp idle.  A search over 2.3 M
+ * particles a few percent of which changed their cell takes 89 us instead of
+ * 134, with the bounds and identities (23 us as kernels of their own) in
+ * this pass.  A cell of more than 128 particles is ordered by one lane. */
+__global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, int np, const int* __restrict__ start, int* part_idx,
+                                                       OrderOutputs out)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int s = __ldg(start + c), e = __ldg(start + c + 1);
-    /* most cells arrive in order (their particles came from one warp):
-     * a read-only pass finds them and leaves them untouched */
-    bool sorted = true;
-    for (int a = s + 1; a < e && sorted; ++a) sorted = part_idx[a - 1] < part_idx[a];
-    if (sorted) return;
-    for (int a = s + 1; a < e; ++a) {
-        const int v = part_idx[a];
-        int b = a - 1;
-        while (b >= s && part_idx[b] > v) {
-            part_idx[b + 1] = part_idx[b];
-            --b;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int first = (blockIdx.x * kBlock + threadIdx.x) & ~31;
+    const int c = first + lane;
+    int s = 0, n = 0;
+    if (c < ncell) {
+        s = __ldg(start + c);
+        n = __ldg(start + c + 1) - s;
+        if (out.beg) {
+            out.beg[c] = n > 0 ? s : -1;
+            out.end[c] = n > 0 ? s + n : -1;
         }
-        part_idx[b + 1] = v;
     }
-}
-
-__global__ void __launch_bounds__(kBlock) k_bounds(int ncell, const int* __restrict__ start, int* __restrict__ beg,
-                                                   int* __restrict__ end)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int s = __ldg(start + c), e = __ldg(start + c + 1);
-    beg[c] = e > s ? s : -1;
-    end[c] = e > s ? e : -1;
+    auto place = [&](int d, int v, int cell) {      /* slot d holds previous slot v's particle */
+        if (out.part_cel) out.part_cel[d] = cell;
+        if (out.ident_out) out.ident_out[d] = lq_in_range(v, np) ? __ldg(out.ident_in + v) : -1;
+    };
+    unsigned todo = __ballot_sync(FULL, n > 0);
+    int k = __ffs((int)todo) - 1;
+    int cs = __shfl_sync(FULL, s, k & 31), cn = __shfl_sync(FULL, n, k & 31);
+    int v = todo && lane < cn ? part_idx[cs + lane] : INT_MAX;
+    while (todo) {
+        todo &= todo - 1;
+        const int k2 = __ffs((int)todo) - 1;
+        const int s2 = __shfl_sync(FULL, s, k2 & 31), n2 = __shfl_sync(FULL, n, k2 & 31);
+        const int v2 = todo && lane < n2 ? part_idx[s2 + lane] : INT_MAX;
+        const int cell = first + k;
+        if (cn <= 32) {
+            const int after = __shfl_down_sync(FULL, v, 1);
+            int r = lane;
+            if (__any_sync(FULL, lane + 1 < cn && v > after)) {
+                r = 0;
+                for (int q = 0; q < cn; ++q) r += __shfl_sync(FULL, v, q) < v;
+                if (lane < cn) part_idx[cs + r] = v;
+            }
+            if (lane < cn) place(cs + r, v, cell);
+        } else if (cn <= 128) {
+            int w[4], r[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                w[u] = 32 * u + lane < cn ? part_idx[cs + 32 * u + lane] : INT_MAX;
+                r[u] = 0;
+            }
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                for (int q = 0; q < 32; ++q) {
+                    const int o = __shfl_sync(FULL, w[b], q);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) r[u] += o < w[u];
+                }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (32 * u + lane < cn) {
+                    part_idx[cs + r[u]] = w[u];
+                    place(cs + r[u], w[u], cell);
+                }
+        } else {
+            if (lane == 0)
+                for (int a = cs + 1; a < cs + cn; ++a) {
+                    const int x = part_idx[a];
+                    int b = a - 1;
+                    while (b >= cs && part_idx[b] > x) {
+                        part_idx[b + 1] = part_idx[b];
+                        --b;
+                    }
+                    part_idx[b + 1] = x;
+                }
+            __syncwarp();
+            for (int d = cs + lane; d < cs + cn; d += 32) place(d, part_idx[d], cell);
+        }
+        k = k2;
+        cs = s2;
+        cn = n2;
+        v = v2;
+    }
 }
 
 __global__ void __launch_bounds__(kBlock) k_gather_f4(int n, const int* __restrict__ idx, const float4* __restrict__ in,
@@ -195,8 +260,38 @@ int scan_scratch_bytes(int ncell, size_t* bytes)
     return LQ_OK;
 }
 
+/* --------------------------------------------- identities of the grids */
+namespace {
+
+struct IdentityRecord {
+    int* ident = nullptr;
+    int* tmp = nullptr;
+    int np = 0;
+    long long gen = 0;
+};
+std::mutex g_id_mu;
+std::unordered_map<const int*, IdentityRecord> g_ids;
+long long g_id_gen = 0;
+
+/* The record that a search over np particles updates (null: none); the
+ * caller holds g_id_mu. */
+IdentityRecord* identity_for_search(const int* key, int np)
+{
+    auto it = g_ids.find(key);
+    if (it == g_ids.end()) return nullptr;
+    IdentityRecord& r = it->second;
+    if (np != r.np) {
+        /* a search over another particle count: identities restart */
+        r.gen = ++g_id_gen;
+        if (np > r.np) return nullptr;
+    }
+    return np > 0 ? &r : nullptr;
+}
+
+}  // namespace
+
 int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, GridBuffers& g, bool bounds,
-                int* health, cudaStream_t s, const float4* idep, const Frames& fr)
+                int* health, cudaStream_t s, const float4* idep, const Frames& fr, const int* identity_key)
 {
     const int np = ph->np, npb = ph->npb, ncell = ph->ncell;
     if (np < 0 || npb < 0 || npb > np || ncell < 1)
@@ -206,7 +301,7 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
                          g.np_cap, g.ncell_cap);
     if (ph->ncell != 2 * ph->ncell_one_layer + 1 || ph->ncell_delete != ncell - 1)
         return set_error(LQ_ERR_ARG, "grid_search: Parameters cell counts are not initialised");
-    LQ_TRY(fill_int(g.count, ncell + 1, 0, s));
+    LQ_TRY_CUDA(cudaMemsetAsync(g.count, 0, sizeof(int) * ((size_t)ncell + 1), s), "cell counts");
     if (np > 0) {
         if (fr.rows && !idep) return set_error(LQ_ERR_ARG, "grid_search: frames need the idep array");
         k_hash_count<<<blocks_for(np), kBlock, 0, s>>>(pd, np, npb, pos, g.key, g.rank, g.count, health, idep, fr);
@@ -214,15 +309,25 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
     }
     size_t bytes = g.scan_bytes;
     LQ_TRY_CUDA(cub::DeviceScan::ExclusiveSum(g.scan_tmp, bytes, g.count, g.start, ncell + 1, s), "cell scan");
+    OrderOutputs out{g.part_cel, bounds ? g.beg : nullptr, bounds ? g.end : nullptr, nullptr, nullptr};
     if (np > 0) {
-        k_scatter<<<blocks_for(np), kBlock, 0, s>>>(np, g.key, g.rank, g.start, g.part_idx, g.part_cel);
+        k_scatter<<<blocks_for(np), kBlock, 0, s>>>(np, g.key, g.rank, g.start, g.part_idx);
         LQ_TRY_CUDA(cudaGetLastError(), "k_scatter");
-        k_cell_order<<<blocks_for(ncell), kBlock, 0, s>>>(ncell, g.start, g.part_idx);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_cell_order");
     }
-    if (bounds) {
-        k_bounds<<<blocks_for(ncell), kBlock, 0, s>>>(ncell, g.start, g.beg, g.end);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_bounds");
+    if (np > 0 || bounds) {
+        std::unique_lock<std::mutex> lock(g_id_mu, std::defer_lock);
+        IdentityRecord* id = nullptr;
+        if (identity_key) {
+            lock.lock();    /* until the launch that follows the identities is queued */
+            id = identity_for_search(identity_key, np);
+        }
+        if (id) {
+            out.ident_in = id->ident;
+            out.ident_out = id->tmp;
+        }
+        k_cell_order<<<blocks_for(ncell), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
+        LQ_TRY_CUDA(cudaGetLastError(), "k_cell_order");
+        if (id) std::swap(id->ident, id->tmp);
     }
     return LQ_OK;
 }
@@ -256,32 +361,12 @@ int bounds_count_grid(unsigned long long* v)
     return LQ_OK;
 }
 
-/* --------------------------------------------- identities of the grids */
 namespace {
-
-struct IdentityRecord {
-    int* ident = nullptr;
-    int* tmp = nullptr;
-    int np = 0;
-    long long gen = 0;
-};
-std::mutex g_id_mu;
-std::unordered_map<const int*, IdentityRecord> g_ids;
-long long g_id_gen = 0;
 
 __global__ void __launch_bounds__(kBlock) k_iota(int n, int* __restrict__ p)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = i;
-}
-
-__global__ void __launch_bounds__(kBlock) k_follow(int n, const int* __restrict__ part_idx,
-                                                   const int* __restrict__ in, int* __restrict__ out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int j = __ldg(part_idx + i);
-    out[i] = lq_in_range(j, n) ? __ldg(in + j) : -1;
 }
 
 }  // namespace
@@ -310,24 +395,6 @@ int identity_reset(const int* key, int np)
         k_iota<<<blocks_for(np), kBlock>>>(np, r.ident);
         LQ_TRY_CUDA(cudaGetLastError(), "k_iota");
     }
-    return LQ_OK;
-}
-
-int identity_after_search(const int* key, const int* part_idx, int np, cudaStream_t s)
-{
-    std::lock_guard<std::mutex> lock(g_id_mu);
-    auto it = g_ids.find(key);
-    if (it == g_ids.end()) return LQ_OK;
-    IdentityRecord& r = it->second;
-    if (np != r.np) {
-        /* a search over another particle count: identities restart */
-        r.gen = ++g_id_gen;
-        if (np > r.np || np <= 0) return LQ_OK;
-    }
-    if (np <= 0) return LQ_OK;
-    k_follow<<<blocks_for(np), kBlock, 0, s>>>(np, part_idx, r.ident, r.tmp);
-    LQ_TRY_CUDA(cudaGetLastError(), "k_follow");
-    std::swap(r.ident, r.tmp);
     return LQ_OK;
 }
 
@@ -451,8 +518,9 @@ extern "C" int lq_grid_neighbor_search(void* grid, const void* par_host, const v
     LqGrid* G = static_cast<LqGrid*>(grid);
     const Parameters* ph = static_cast<const Parameters*>(par_host);
     LQ_TRY(lqb::grid_search(ph, static_cast<const Parameters*>(par_device), reinterpret_cast<const float4*>(pospres),
-                            G->g, true, nullptr, static_cast<cudaStream_t>(stream)));
-    return lqb::identity_after_search(G->g.beg, G->g.part_idx, ph->np, static_cast<cudaStream_t>(stream));
+                            G->g, true, nullptr, static_cast<cudaStream_t>(stream), nullptr, lqb::Frames(),
+                            G->g.beg));
+    return LQ_OK;
 }
 
 extern "C" int lq_grid_arrays(void* grid, const int** part_cel, const int** part_idx, const int** cell_beg,
@@ -596,8 +664,9 @@ void LoquatGrid::NeighborSearch(Parameters* par_host, Parameters* par_device, fl
     g.part_cel = part_cel;
     g.beg = cell_beg;
     g.end = cell_end;
-    if (lqb::grid_search(par_host, par_device, pospres, g, true, nullptr, 0) != LQ_OK) die("NeighborSearch");
-    if (lqb::identity_after_search(cell_beg, part_idx, par_host->np, 0) != LQ_OK) die("NeighborSearch");
+    if (lqb::grid_search(par_host, par_device, pospres, g, true, nullptr, 0, nullptr, lqb::Frames(), cell_beg) !=
+        LQ_OK)
+        die("NeighborSearch");
 }
 
 void LoquatGrid::SortArrayFloat4(int np, float4* data, float4* data_cache)

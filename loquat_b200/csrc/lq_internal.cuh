@@ -105,7 +105,7 @@ struct GridBuffers {
     int* count = nullptr;     /* particles per cell             ncell + 1 */
     int* start = nullptr;     /* exclusive scan of count        ncell + 1 */
     int* part_idx = nullptr;  /* sorted slot -> previous slot   np */
-    int* part_cel = nullptr;  /* sorted key                     np */
+    int* part_cel = nullptr;  /* optional sorted key            np */
     int* beg = nullptr;       /* optional per-cell bounds       ncell */
     int* end = nullptr;
     void* scan_tmp = nullptr;
@@ -121,10 +121,12 @@ int bounds_count_sph(unsigned long long* v);
 
 /* Hash, count, scan, scatter and in-cell ordering: a stable sort of the
  * particles by cell key.  Writes key, rank, count, start, part_idx,
- * part_cel, and beg/end when `bounds` is set.  `health` may be null. */
+ * part_cel, and beg/end when `bounds` is set.  `health` may be null.  With
+ * identity_key (a grid's cell_beg) the identities of that grid's particles
+ * follow the search. */
 int grid_search(const Parameters* par_host, const Parameters* par_dev, const float4* pos, GridBuffers& g,
                 bool bounds, int* health, cudaStream_t s, const float4* idep = nullptr,
-                const Frames& fr = Frames());
+                const Frames& fr = Frames(), const int* identity_key = nullptr);
 
 /* Particle identities of the drop-in grids (lq_grid_* and LoquatGrid),
  * keyed by the grid's cell_beg array: ident[slot] is the slot the particle
@@ -140,7 +142,6 @@ struct GridIdentity {
     long long gen = 0;
 };
 int identity_reset(const int* key, int np);
-int identity_after_search(const int* key, const int* part_idx, int np, cudaStream_t s);
 void identity_release(const int* key);
 bool identity_find(const int* key, GridIdentity* out);
 

@@ -755,7 +755,6 @@ int create(LqSim* S, const Parameters* par, const float* pos, const float* vel, 
     LQ_TRY(dev_alloc(S, (void**)&g.key, n * sizeof(int)));
     LQ_TRY(dev_alloc(S, (void**)&g.rank, n * sizeof(int)));
     LQ_TRY(dev_alloc(S, (void**)&g.part_idx, n * sizeof(int)));
-    LQ_TRY(dev_alloc(S, (void**)&g.part_cel, n * sizeof(int)));
     LQ_TRY(dev_alloc(S, (void**)&g.count, sizeof(int) * (size_t)(ncell + 1)));
     LQ_TRY(dev_alloc(S, (void**)&g.start, sizeof(int) * (size_t)(ncell + 1)));
     LQ_TRY(dev_alloc(S, &g.scan_tmp, g.scan_bytes));
@@ -1532,12 +1531,11 @@ extern "C" int lq_sim_rebuild_launches(void* sim, int* launches)
 {
     if (!sim || !launches) return lqb::set_error(LQ_ERR_ARG, "lq_sim_rebuild_launches: null argument");
     LqSim* S = static_cast<LqSim*>(sim);
-    /* count reset, hash, scatter, cell order (the scan is a library
-     * kernel), gather, copy, material list and its order (when npm > 0),
+    /* hash, scatter, cell order (the scan is a library kernel), gather, copy, material list and its order (when npm > 0),
      * boundary list (when npb > 0),
      * full pack of the neighbour data, tile segments and fill (tiled
      * shapes; their scan is a library kernel) */
-    *launches = 4 + 1 + 1 + (S->npm > 0 ? 2 : 0) + (S->npb > 0 ? 1 : 0) + 1 + (tiled(S) && S->npm > 0 ? 2 : 0);
+    *launches = 3 + 1 + 1 + (S->npm > 0 ? 2 : 0) + (S->npb > 0 ? 1 : 0) + 1 + (tiled(S) && S->npm > 0 ? 2 : 0);
     /* with two-level lists the lists the stages read are renewed from the
      * wide ones right after */
     int renewal = 0;
