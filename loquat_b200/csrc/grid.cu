@@ -108,7 +108,7 @@ struct OrderOutputs {
     int* ident_out;
 };
 
-/* A warp takes 32 cells, one after the other: the lanes load a cell's slots
+/* A warp takes kCells cells, one after the other: the lanes load a cell's slots
  * (the next cell's meanwhile), a vote tells whether they are in order, and
  * if not each lane finds its particle's place by counting the smaller ones.
  * One thread per cell, inserting, was a chain of about 17 dependent loads
@@ -116,15 +116,16 @@ struct OrderOutputs {
  * particles a few percent of which changed their cell takes 89 us instead of
  * 134, with the bounds and identities (23 us as kernels of their own) in
  * this pass.  A cell of more than 128 particles is ordered by one lane. */
+template <int kCells>
 __global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, int np, const int* __restrict__ start, int* part_idx,
                                                        OrderOutputs out)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int first = (blockIdx.x * kBlock + threadIdx.x) & ~31;
+    const int first = (blockIdx.x * kBlock + threadIdx.x) / 32 * kCells;
     const int c = first + lane;
     int s = 0, n = 0;
-    if (c < ncell) {
+    if (lane < kCells && c < ncell) {
         s = __ldg(start + c);
         n = __ldg(start + c + 1) - s;
         if (out.beg) {
@@ -206,16 +207,13 @@ __global__ void __launch_bounds__(kBlock) k_gather_f4(int n, const int* __restri
     if (lq_in_range(j, n)) out[i] = __ldg(in + j);
 }
 
-/* tensor2d as three float2 words: consecutive threads write consecutive words. */
-__global__ void __launch_bounds__(kBlock) k_gather_t2(int n, const int* __restrict__ idx, const float2* __restrict__ in,
-                                                      float2* __restrict__ out)
+__global__ void __launch_bounds__(kBlock) k_gather_t2(int n, const int* __restrict__ idx, const tensor2d* __restrict__ in,
+                                                      tensor2d* __restrict__ out)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3LL * n) return;
-    const int i = (int)(t / 3);
-    const int w = (int)(t - 3LL * i);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
     const int j = __ldg(idx + i);
-    if (lq_in_range(j, n)) out[t] = __ldg(in + 3LL * j + w);
+    if (lq_in_range(j, n)) store_t2(out, i, load_t2(in, j));
 }
 
 __global__ void __launch_bounds__(kBlock) k_gather_state(int n, const int* __restrict__ idx, State in, State out)
@@ -325,7 +323,12 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
             out.ident_in = id->ident;
             out.ident_out = id->tmp;
         }
-        k_cell_order<<<blocks_for(ncell), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
+        /* few cells: fewer per warp, whose chain of cells is the time
+         * (15 k cells: 6.0 us a launch with 8, 12.3 with 32) */
+        if (ncell <= 1 << 18)
+            k_cell_order<8><<<blocks_for(ncell, kBlock / 4), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
+        else
+            k_cell_order<32><<<blocks_for(ncell), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
         LQ_TRY_CUDA(cudaGetLastError(), "k_cell_order");
         if (id) std::swap(id->ident, id->tmp);
     }
@@ -343,8 +346,7 @@ int gather_float4(int n, const int* idx, const float4* in, float4* out, cudaStre
 int gather_tensor2d(int n, const int* idx, const tensor2d* in, tensor2d* out, cudaStream_t s)
 {
     if (n <= 0) return LQ_OK;
-    k_gather_t2<<<blocks_for(3LL * n), kBlock, 0, s>>>(n, idx, reinterpret_cast<const float2*>(in),
-                                                        reinterpret_cast<float2*>(out));
+    k_gather_t2<<<blocks_for(n), kBlock, 0, s>>>(n, idx, in, out);
     LQ_TRY_CUDA(cudaGetLastError(), "k_gather_t2");
     return LQ_OK;
 }

@@ -193,15 +193,13 @@ struct StageOps {
  * sigma/rho^2: 52 bytes per particle, 48 in the compensated form, whose
  * velocity is packed into two words) that the pair kernel gathers; with
  * `pack` they are packed from the state first, in the form of
- * `compensated`.  With `rows` (thread-per-target shapes, `pack` set)
- * target t reads list row rows[t] (-1: walk the stencil), whose entries
- * index records packed in another slot order: slot i's record goes to
- * map[i], target t's own at npb + rows[t]. */
+ * `compensated`.  With `rows` (thread-per-target shapes, no `pack`) target t
+ * reads list row rows[t] (-1: walk the stencil), whose entries index records
+ * packed in another slot order, target t's own at npb + rows[t]. */
 int launch_interaction_list(const Parameters* par_host, const Parameters* par_dev, const State& st, const Rates& r,
                             const Cells& c, const NeighborList& nl, cudaStream_t s, const Frames& fr = Frames(),
                             bool compensated = false, float* rec = nullptr, int shape = 0, bool pack = true,
-                            const int* order = nullptr, const int* rows = nullptr, const int* map = nullptr,
-                            const StageOps* ops = nullptr);
+                            const int* order = nullptr, const int* rows = nullptr, const StageOps* ops = nullptr);
 /* Whether a launch shape integrates its targets when asked to (ops); the
  * warp-cooperative ones store their rates for the integrator kernels.  The
  * thread-per-target shapes store rates in the plain form only. */
@@ -210,7 +208,7 @@ bool integrates_in_pair_kernel(int shape);
  * packed_velocity selects the compensated pair kernel's record.  The slots
  * below n2 are packed into rec2 as well. */
 int launch_pack_neighbors(const Parameters* par_host, const State& st, float* rec, int first, cudaStream_t s,
-                          bool packed_velocity, const int* map = nullptr, float* rec2 = nullptr, int n2 = 0);
+                          bool packed_velocity, float* rec2 = nullptr, int n2 = 0);
 /* Adami over the boundary lists reading the packed arrays (material slots
  * packed), writing the boundary stress into the state, into str2 when set
  * and into the stress words of the packed arrays (the boundary slots'

@@ -409,7 +409,7 @@ int enqueue_interaction(LqSim* S, int stage, cudaStream_t s)
     ops.keep_rates = !first && (S->flags & LQ_SIM_DYNAMIC_DT);
     return lqb::launch_interaction_list(&S->ph, S->pd, first ? S->S : S->S2, S->R, cells, S->nlm, s, S->fr,
                                         S->flags & LQ_SIM_MIXED, first ? S->rec : S->rec2, S->pair_shape, false,
-                                        tile_order(S), nullptr, nullptr,
+                                        tile_order(S), nullptr,
                                         lqb::integrates_in_pair_kernel(S->pair_shape) ? &ops : nullptr);
 }
 
@@ -455,7 +455,7 @@ int enqueue_rebuild(LqSim* S, cudaStream_t s)
     LQ_TRY(build_lists(S, s));
     /* every slot's packed neighbour data (the boundary slots keep theirs,
      * in both stages' arrays, until the next build) */
-    LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, nullptr, S->rec2, S->npb));
+    LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, S->rec2, S->npb));
     return lqb::launch_tile_order(ph, S->g.start, S->pair_shape, S->tile, s);
 }
 
@@ -1608,7 +1608,7 @@ int profiled_step(LqSim* S, PhaseTimer& T)
         LQ_TRY(T.close(s));
         LQ_TRY(T.mark(s, PH_LIST));
         LQ_TRY(build_lists(S, s));
-        LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, nullptr, S->rec2, S->npb));
+        LQ_TRY(lqb::launch_pack_neighbors(ph, S->S, S->rec, 0, s, S->flags & LQ_SIM_MIXED, S->rec2, S->npb));
         LQ_TRY(lqb::launch_tile_order(ph, S->g.start, S->pair_shape, S->tile, s));
         LQ_TRY(T.close(s));
     }

@@ -560,25 +560,18 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
     }
 }
 
-/* Slot i's packed record, at i or (with map) at map[i], the index lists
- * of another slot order gather it at (slots with none are skipped); the
- * slots below n2 also into nb2. */
+/* Slot i's packed record; the slots below n2 also into nb2. */
 template <bool kPk>
 __global__ void __launch_bounds__(kBlock) k_pack_neighbors(int first, int np, State st, NbrArrays nb,
-                                                           const int* __restrict__ map, NbrArrays nb2, int n2)
+                                                           NbrArrays nb2, int n2)
 {
     const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    int o = i;
-    if (map) {
-        o = __ldg(map + i);
-        if ((unsigned)o >= (unsigned)np) return;
-    }
     const float4 x = __ldg(st.pos + i);
     const float4 v = __ldg(st.vel + i);
     const tensor2d s = load_t2(st.str, i);
-    pack_slot<kPk>(nb, o, x, v, s);
-    if (i < n2) pack_slot<kPk>(nb2, o, x, v, s);
+    pack_slot<kPk>(nb, i, x, v, s);
+    if (i < n2) pack_slot<kPk>(nb2, i, x, v, s);
 }
 
 /* A list entry: each 128-byte row of a list is read once per launch, so it
@@ -1060,8 +1053,9 @@ struct CellSums {
 __device__ __forceinline__ bool cell_range(const Cells& c, int cell, int& s, int& e)
 {
     s = __ldg(c.beg + cell);
+    if (s == -1) return false;
     e = __ldg(c.end + cell);
-    return s != -1;
+    return true;
 }
 
 /* The whole warp calls it, its four groups in step (votes and loops are the
@@ -1135,17 +1129,22 @@ __device__ __forceinline__ CellSums sum_material_cells(const Parameters* __restr
         const int X = cx + col % 3 - 1, Y = cy + col / 3 - 1;
         int s = 0, e = 0;
         bool apart = false;
-        if (col < 9 && X >= 0 && X < nx && Y >= 0 && Y < ny)
-            for (int z = zlo; z <= zhi; ++z) {
-                int b, f;
-                if (!cell_range(cells, L + (X * ny + Y) * nz + z, b, f)) continue;
+        if (col < 9 && X >= 0 && X < nx && Y >= 0 && Y < ny) {
+            const int cell = L + (X * ny + Y) * nz + zlo;
+            int b[3];
+#pragma unroll
+            for (int z = 0; z < 3; ++z) b[z] = zlo + z <= zhi ? __ldg(cells.beg + cell + z) : -1;
+#pragma unroll
+            for (int z = 0; z < 3; ++z) {
+                if (b[z] == -1) continue;
                 if (e == 0) {
-                    s = b;
-                } else if (b != e) {
+                    s = b[z];
+                } else if (b[z] != e) {
                     apart = true;
                 }
-                e = f;
+                e = __ldg(cells.end + cell + z);
             }
+        }
         const bool any_apart = __any_sync(FULL, apart);
         for (int c = 0; c < kCellLanes && first + c < 9; ++c) {
             const int cs = __shfl_sync(FULL, s, c, kCellLanes), ce = __shfl_sync(FULL, e, c, kCellLanes);
@@ -1737,16 +1736,16 @@ int launch_list_arrange(int n, const NeighborList& nl, cudaStream_t s)
 }
 
 int launch_pack_neighbors(const Parameters* ph, const State& st, float* rec, int first, cudaStream_t s,
-                          bool packed_velocity, const int* map, float* rec2, int n2)
+                          bool packed_velocity, float* rec2, int n2)
 {
     const int n = ph->np - first;
     if (n <= 0) return LQ_OK;
     const NbrArrays nb = nbr_arrays(rec, ph->np);
     const NbrArrays nb2 = rec2 ? nbr_arrays(rec2, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     if (packed_velocity)
-        k_pack_neighbors<true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map, nb2, n2);
+        k_pack_neighbors<true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, nb2, n2);
     else
-        k_pack_neighbors<false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, map, nb2, n2);
+        k_pack_neighbors<false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(first, ph->np, st, nb, nb2, n2);
     LQ_TRY_CUDA(cudaGetLastError(), "k_pack_neighbors");
     return LQ_OK;
 }
@@ -1870,7 +1869,7 @@ bool integrates_in_pair_kernel(int shape) { return shape != 5 && shape != 6; }
 int launch_interaction_list(const Parameters* ph, const Parameters* pd, const State& st, const Rates& r,
                             const Cells& c, const NeighborList& nl, cudaStream_t s, const Frames& fr,
                             bool compensated, float* rec, int shape, bool pack, const int* order,
-                            const int* rows, const int* map, const StageOps* ops)
+                            const int* rows, const StageOps* ops)
 {
     if (ph->npm <= 0) return LQ_OK;
     if (!rec) return set_error(LQ_ERR_ARG, "interaction: the packed neighbour arrays are required");
@@ -1878,10 +1877,10 @@ int launch_interaction_list(const Parameters* ph, const Parameters* pd, const St
         return set_error(LQ_ERR_ARG, "interaction: packed neighbour arrays must be 32-byte aligned");
     if (shape < 0 || shape >= kPairShapeCount) return set_error(LQ_ERR_ARG, "interaction: launch shape %d", shape);
     const NbrArrays nb = nbr_arrays(rec, ph->np);
-    if (rows && (!map || !pack || ops || shape == 5 || shape == 6))
-        return set_error(LQ_ERR_ARG, "interaction: list rows need a record map, a pack and a thread-per-target "
-                         "shape that stores its rates");
-    if (pack) LQ_TRY(launch_pack_neighbors(ph, st, rec, 0, s, compensated, rows ? map : nullptr));
+    if (rows && (pack || ops || shape == 5 || shape == 6))
+        return set_error(LQ_ERR_ARG, "interaction: list rows need records packed in their order and a "
+                         "thread-per-target shape that stores its rates");
+    if (pack) LQ_TRY(launch_pack_neighbors(ph, st, rec, 0, s, compensated));
     if (kPairShapes[shape][2] == 1 && !order)
         return set_error(LQ_ERR_ARG, "interaction: launch shape %d needs the tile order", shape);
     if (kPairShapes[shape][2] != 1) order = nullptr;
@@ -1951,37 +1950,33 @@ lqb::State state_of(const float* pos, const float* vel, const float* idep, const
 
 namespace {
 
-/* Launch shape of the drop-in interaction's pair kernel (lqb::kPairShapes). */
-constexpr int kDropInShape = 9;
+/* Launch shape of the drop-in interaction's pair kernel (lqb::kPairShapes):
+ * slot order, since each search moves the slots and the tile order would be
+ * made anew for every call: the launch takes 308 us at 786 k targets either
+ * way, and the tile order took 50. */
+constexpr int kDropInShape = 0;
 /* Skin of the drop-in interaction's lists (of h) when the caller's grid
  * tracks particle identities: the lists then hold every pair within
  * 2h + skin and are carried across calls until some particle has moved
  * half the skin. */
 constexpr float kDropInSkinOverH = 0.05f;
 
-/* Working arrays of the drop-in interaction, one set per device: the cell
- * starts derived from the caller's cell_beg / cell_end, the pair kernel's
- * tile order with its scratch, the neighbour lists
- * and the packed neighbour data.  lq_interaction_reserve sizes them from a
+/* Working arrays of the drop-in interaction, one set per device: the
+ * neighbour lists, the packed neighbour data and what carries both from
+ * call to call.  lq_interaction_reserve sizes them from a
  * Parameters record (the drop-in LoquatGrid's GridConfig calls it, where
  * the reference allocates its arrays); a call that needs more than was
  * reserved grows them itself, synchronising the device before the old
  * arrays are freed.  Calls that overlap on the GPU share the arrays and
  * must not. */
 struct DropInWorkspace {
-    int np = 0, ncell = 0, nseg = 0, npm = 0;
-    int* start = nullptr;           /* ncell + 1 cell starts */
-    int* counts = nullptr;          /* ncell + 1 particles per cell */
-    void* scan_tmp = nullptr;       /* cell-start scan */
-    size_t scan_bytes = 0;
-    lqb::TileOrder to;              /* tile order and its segment scratch */
+    int np = 0, npm = 0;
     lqb::NeighborList nl;           /* material targets' lists */
     float* rec = nullptr;           /* packed neighbour data, 13 floats per particle */
     /* lists carried across calls (caller grids that track identities) */
     float4* xbuild = nullptr;       /* np: positions at the build, by identity */
     int* build_of = nullptr;        /* np: identity -> slot at the build */
     int* rows = nullptr;            /* npm: target -> its list's row (the target's slot at the build) */
-    int* pidx = nullptr;            /* np: slot -> its particle's slot at the build (its record's index) */
     int* moved = nullptr;           /* device flag: a particle moved half the skin since the build */
     int* tally = nullptr;           /* device counts of [0] builds and [1] reuses of carried lists */
     const int* key = nullptr;       /* the grid (its cell_beg) the carried lists belong to */
@@ -2009,15 +2004,11 @@ int ws_alloc(DropInWorkspace& w, void** p, size_t bytes)
     return LQ_OK;
 }
 
-/* Sizes every array for the Parameters' particle and cell counts. */
+/* Sizes every array for the Parameters' particle counts. */
 int size_workspace(DropInWorkspace& w, const Parameters* ph)
 {
-    const int np = ph->np > 1 ? ph->np : 1, ncell = ph->ncell, npm = ph->npm > 1 ? ph->npm : 1;
-    int nseg = 0;
-    size_t seg_scan = 0, cell_scan = 0;
-    LQ_TRY(lqb::tile_order_scratch(ph, &nseg, &seg_scan));
-    LQ_TRY(lqb::scan_scratch_bytes(ncell, &cell_scan));
-    if (np <= w.np && ncell <= w.ncell && nseg <= w.nseg && npm <= w.npm && w.rec) return LQ_OK;
+    const int np = ph->np > 1 ? ph->np : 1, npm = ph->npm > 1 ? ph->npm : 1;
+    if (np <= w.np && npm <= w.npm && w.rec) return LQ_OK;
     if (!w.allocs.empty()) LQ_TRY_CUDA(cudaDeviceSynchronize(), "interaction workspace");
     long long rebuilds = w.rebuilds, reuses = w.reuses;
     if (w.tally) {
@@ -2034,23 +2025,13 @@ int size_workspace(DropInWorkspace& w, const Parameters* ph)
     auto A = [&](void** p, size_t bytes) {
         if (st == LQ_OK) st = ws_alloc(n, p, bytes);
     };
-    A((void**)&n.start, sizeof(int) * ((size_t)ncell + 1));
-    A((void**)&n.counts, sizeof(int) * ((size_t)ncell + 1));
-    A(&n.scan_tmp, cell_scan);
-    n.scan_bytes = cell_scan;
-    A((void**)&n.to.seg, sizeof(int) * 3 * (size_t)nseg);
-    A(&n.to.scan_tmp, seg_scan);
-    n.to.nseg_cap = nseg;
-    n.to.scan_bytes = seg_scan;
     A((void**)&n.rec, sizeof(float) * 13 * (size_t)np);
     n.nl.stride = (npm + 31) / 32 * 32;
     A((void**)&n.nl.list, sizeof(int) * (size_t)LQ_NBR_CAP * n.nl.stride);
     A((void**)&n.nl.count, sizeof(int) * (size_t)n.nl.stride);
-    A((void**)&n.to.order, sizeof(int) * (size_t)npm);
     A((void**)&n.xbuild, sizeof(float4) * (size_t)np);
     A((void**)&n.build_of, sizeof(int) * (size_t)np);
     A((void**)&n.rows, sizeof(int) * (size_t)npm);
-    A((void**)&n.pidx, sizeof(int) * (size_t)np);
     A((void**)&n.moved, sizeof(int));
     A((void**)&n.tally, 2 * sizeof(int));
     if (st == LQ_OK) {
@@ -2062,8 +2043,6 @@ int size_workspace(DropInWorkspace& w, const Parameters* ph)
         return st;
     }
     n.np = np;
-    n.ncell = ncell;
-    n.nseg = nseg;
     n.npm = npm;
     w = std::move(n);
     return LQ_OK;
@@ -2088,7 +2067,7 @@ int dropin_workspace(const Parameters* ph, DropInWorkspace** out)
  * neighbour record at its build slot, so the pair kernel gathers through
  * the stored entries as they are, each target reading the row of its build
  * slot; a later call whose particles have all moved less than half the
- * skin only maps slots to build slots (k_record_index).  The records stay
+ * skin only maps slots to build slots (k_carry).  The records stay
  * in the cell order of the build. */
 __global__ void __launch_bounds__(256) k_moved_half_skin(int np, const float4* __restrict__ pos,
                                                          const int* __restrict__ ident,
@@ -2107,57 +2086,35 @@ __global__ void __launch_bounds__(256) k_moved_half_skin(int np, const float4* _
     if (far) *moved = 1;
 }
 
-/* The call's decision, counted: a build when a particle moved (or nothing
- * was carried), else a reuse. */
-__global__ void k_tally_decision(const int* __restrict__ moved, int* __restrict__ tally)
-{
-    tally[*moved ? 0 : 1] += 1;
-}
-
-/* Each slot's record index, the build slot of its particle (-1 when its
- * particle has none), and each material target's list row (its record
- * index less npb; -1: no carried list, the pair kernel walks its
- * stencil). */
-__global__ void __launch_bounds__(256) k_record_index(int np, int npb, const int* __restrict__ ident,
-                                                      const int* __restrict__ build_of, int* __restrict__ pidx,
-                                                      int* __restrict__ rows)
+/* What a call does per slot besides its lists: a build (*moved, or moved
+ * null) is recorded, each particle's build slot and position by identity;
+ * the particle's neighbour record is packed at its build slot (not for a
+ * particle that has none); and each material target gets its list's row,
+ * that slot less npb (-1: no carried list, the pair kernel walks its
+ * stencil).  One thread counts the decision. */
+__global__ void __launch_bounds__(256) k_carry(int np, int npb, lqb::State st, const int* __restrict__ ident,
+                                               const int* __restrict__ moved, float4* __restrict__ xbuild,
+                                               int* __restrict__ build_of, lqb::NbrArrays nb, int* __restrict__ rows,
+                                               int* __restrict__ tally)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= np) return;
+    const bool build = !moved || *moved;
+    if (c == 0) tally[build ? 0 : 1] += 1;
     const int id = __ldg(ident + c);
-    const int b = (unsigned)id < (unsigned)np ? __ldg(build_of + id) : -1;
-    const int o = (unsigned)b < (unsigned)np ? b : -1;
-    pidx[c] = o;
-    if (c >= npb) rows[c - npb] = o >= npb ? o - npb : -1;
-}
-
-/* A build recorded for carrying (skipped unless *moved): each particle's
- * build slot and position, by identity. */
-__global__ void __launch_bounds__(256) k_store_build(int np, const int* __restrict__ ident,
-                                                     const float4* __restrict__ pos, float4* __restrict__ xbuild,
-                                                     int* __restrict__ build_of, const int* __restrict__ moved)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= np || !*moved) return;
-    const int id = __ldg(ident + c);
+    const float4 x = __ldg(st.pos + c);
+    int o = -1;
     if ((unsigned)id < (unsigned)np) {
-        xbuild[id] = __ldg(pos + c);
-        build_of[id] = c;
+        if (build) {
+            xbuild[id] = x;
+            build_of[id] = o = c;
+        } else {
+            o = build_of[id];
+            if ((unsigned)o >= (unsigned)np) o = -1;
+        }
     }
-}
-
-/* Particles per cell from the reference's per-cell bounds (-1: empty). */
-__global__ void __launch_bounds__(256) k_cell_counts(int ncell, const int* __restrict__ beg,
-                                                     const int* __restrict__ end, int* __restrict__ counts)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > ncell) return;
-    int n = 0;
-    if (c < ncell) {
-        const int b = __ldg(beg + c);
-        n = b == -1 ? 0 : __ldg(end + c) - b;
-    }
-    counts[c] = n;
+    if (c >= npb) rows[c - npb] = o >= npb ? o - npb : -1;
+    if (o >= 0) lqb::pack_slot<false>(nb, o, x, __ldg(st.vel + c), lqb::load_t2(st.str, c));
 }
 
 }  // namespace
@@ -2197,11 +2154,10 @@ extern "C" int lq_interaction_reserve(const void* par_host)
 
 /* The reference's ParticleInteraction (src/particle_interaction.h:27-40).
  * The caller's grid (cell_beg / cell_end: every particle sorted into its
- * cell, cells in key order) gives the cell starts; the material targets
- * are ordered into compact tiles, their neighbours within 2h are found by
- * the 27-cell walk in the reference's visiting order into lists, and the
- * pair kernel sums over the lists from the packed neighbour data, in plain
- * FP32 as the reference computes. */
+ * cell, cells in key order) gives the material targets' neighbours within
+ * 2h, found by the 27-cell walk into lists, and the pair kernel sums over
+ * the lists from the packed neighbour data, in plain FP32 as the reference
+ * computes. */
 extern "C" int lq_particle_interaction(const void* par_host, const void* par_device, const float* pospres,
                                        const float* velrhop, const float* idep, const float* str, const float* stn,
                                        float* accad, float* spin, float* acestn, const int* cell_beg,
@@ -2218,52 +2174,42 @@ extern "C" int lq_particle_interaction(const void* par_host, const void* par_dev
     const lqb::State st = state_of(pospres, velrhop, idep, str, stn);
     DropInWorkspace* w = nullptr;
     LQ_TRY(dropin_workspace(ph, &w));
-    const int ncell = ph->ncell;
-    k_cell_counts<<<(ncell + 256) / 256, 256, 0, s>>>(ncell, cell_beg, cell_end, w->counts);
-    LQ_TRY_CUDA(cudaGetLastError(), "k_cell_counts");
-    size_t bytes = w->scan_bytes;
-    LQ_TRY_CUDA(cub::DeviceScan::ExclusiveSum(w->scan_tmp, bytes, w->counts, w->start, ncell + 1, s),
-                "cell start scan");
-    const lqb::Cells c{w->start, nullptr, nullptr};
+    const lqb::Cells c{nullptr, cell_beg, cell_end};
     const int np = ph->np, npb = ph->npb, npm = ph->npm;
     const int nb256 = (np + 255) / 256;
     lqb::GridIdentity gi;
     if (lqb::identity_find(cell_beg, &gi) && gi.np == np) {
         /* the caller's grid tracks its particles: carry the lists while
          * every particle stays within half the skin of its build position.
-         * The device decides (no host synchronisation): both paths are
-         * enqueued and the one not taken returns at once. */
+         * The device decides (no host synchronisation): the list build is
+         * enqueued and returns at once when it is not taken. */
         const float skin = kDropInSkinOverH * ph->h;
         const bool carried =
             w->built && w->key == cell_beg && w->gen == gi.gen && w->np_built == np && w->npb_built == npb;
+        const int* moved = nullptr;
         if (carried) {
             LQ_TRY_CUDA(cudaMemsetAsync(w->moved, 0, sizeof(int), s), "moved flag");
             k_moved_half_skin<<<nb256, 256, 0, s>>>(np, st.pos, gi.ident, w->xbuild, 0.25f * skin * skin, w->moved);
             LQ_TRY_CUDA(cudaGetLastError(), "k_moved_half_skin");
-        } else {
-            LQ_TRY(lqb::fill_int(w->moved, 1, 1, s));
+            moved = w->moved;
         }
-        k_tally_decision<<<1, 1, 0, s>>>(w->moved, w->tally);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_tally_decision");
-        /* a build (skipped unless moved): fresh lists in the current
-         * slots, kept with each particle's build slot and position */
+        /* a build: fresh lists in the current slots, kept with each
+         * particle's build slot and position */
         LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, npb, npm, 0, 2.0f * ph->h + skin, st.pos, c, w->nl, nullptr,
-                                               s, nullptr, lqb::Frames(), nullptr, 0.0f, w->moved));
-        k_store_build<<<nb256, 256, 0, s>>>(np, gi.ident, st.pos, w->xbuild, w->build_of, w->moved);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_store_build");
+                                               s, nullptr, lqb::Frames(), nullptr, 0.0f, moved));
+        /* either way the pair kernel reads the lists of the last build,
+         * each target at the row of its build slot, with the records
+         * packed at the build slots: a reuse maps only slots */
+        k_carry<<<nb256, 256, 0, s>>>(np, npb, st, gi.ident, moved, w->xbuild, w->build_of,
+                                      lqb::nbr_arrays(w->rec, np), w->rows, w->tally);
+        LQ_TRY_CUDA(cudaGetLastError(), "k_carry");
         w->built = true;
         w->key = cell_beg;
         w->gen = gi.gen;
         w->np_built = np;
         w->npb_built = npb;
-        /* either way the pair kernel reads the lists of the last build,
-         * each target at the row of its build slot, with the records
-         * packed at the build slots: a reuse maps only slots */
-        k_record_index<<<nb256, 256, 0, s>>>(np, npb, gi.ident, w->build_of, w->pidx, w->rows);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_record_index");
-        LQ_TRY(lqb::launch_tile_order(ph, w->start, kDropInShape, w->to, s));
         return lqb::launch_interaction_list(ph, pd, st, r, c, w->nl, s, lqb::Frames(), false, w->rec, kDropInShape,
-                                            true, w->to.order, w->rows, w->pidx);
+                                            false, nullptr, w->rows);
     }
     /* a grid of the caller's own: lists built in its slots at every call,
      * with the pair body's own cut-off test (q < 2 with the candidate
@@ -2271,9 +2217,7 @@ extern "C" int lq_particle_interaction(const void* par_host, const void* par_dev
     const float cut = 2.0f * ph->h * sqrtf(1.0001f);
     LQ_TRY(lqb::launch_neighbor_list_range(ph, pd, npb, npm, 0, cut, st.pos, c, w->nl, nullptr, s));
     w->built = false;
-    LQ_TRY(lqb::launch_tile_order(ph, w->start, kDropInShape, w->to, s));
-    return lqb::launch_interaction_list(ph, pd, st, r, c, w->nl, s, lqb::Frames(), false, w->rec, kDropInShape, true,
-                                        w->to.order);
+    return lqb::launch_interaction_list(ph, pd, st, r, c, w->nl, s, lqb::Frames(), false, w->rec, kDropInShape, true);
 }
 
 extern "C" int lq_adami_boundary(const void* par_host, const void* par_device, const float* pospres,
