@@ -113,7 +113,7 @@ struct OrderOutputs {
  * if not each lane finds its particle's place by counting the smaller ones.
  * One thread per cell, inserting, was a chain of about 17 dependent loads
  * and stores with most threads of a warp idle.  A search over 2.3 M
- * particles a few percent of which changed their cell takes 89 us instead of
+ * particles a few percent of which changed their cell takes 83 us instead of
  * 134, with the bounds and identities (23 us as kernels of their own) in
  * this pass.  A cell of more than 128 particles is ordered by one lane. */
 template <int kCells>
@@ -324,11 +324,12 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
             out.ident_out = id->tmp;
         }
         /* few cells: fewer per warp, whose chain of cells is the time
-         * (15 k cells: 6.0 us a launch with 8, 12.3 with 32) */
+         * (15 k cells: 6.0 us a launch with 8, 12.3 with 32; 2.1 M cells:
+         * 83 us a search with 16, 86 with 8, 90 with 32) */
         if (ncell <= 1 << 18)
             k_cell_order<8><<<blocks_for(ncell, kBlock / 4), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
         else
-            k_cell_order<32><<<blocks_for(ncell), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
+            k_cell_order<16><<<blocks_for(ncell, kBlock / 2), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
         LQ_TRY_CUDA(cudaGetLastError(), "k_cell_order");
         if (id) std::swap(id->ident, id->tmp);
     }
