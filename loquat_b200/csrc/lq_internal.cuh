@@ -210,15 +210,13 @@ bool integrates_in_pair_kernel(int shape);
 int launch_pack_neighbors(const Parameters* par_host, const State& st, float* rec, int first, cudaStream_t s,
                           bool packed_velocity, float* rec2 = nullptr, int n2 = 0);
 /* Adami over the boundary lists reading the packed arrays (material slots
- * packed), writing the boundary stress into the state, into str2 when set
- * and into the stress words of the packed arrays (the boundary slots'
- * other words, from the last full pack, stay), those of rec2 too when it is
- * set.  With act / nact (device;
- * from launch_boundary_targets; act holds at least npb ints) only the
- * slots act[0 .. *nact) are visited. */
+ * packed), writing the boundary stress into the state and str2 and into the
+ * stress words of the packed arrays rec and rec2 (the boundary slots' other
+ * words, from the last full pack, stay), for the slots act[0 .. *nact)
+ * (device; from launch_boundary_targets). */
 int launch_adami_packed(const Parameters* par_host, const Parameters* par_dev, const State& st,
-                        const NeighborList& nl, float* rec, cudaStream_t s, tensor2d* str2 = nullptr,
-                        float* rec2 = nullptr, const int* act = nullptr, const int* nact = nullptr);
+                        const NeighborList& nl, float* rec, cudaStream_t s, tensor2d* str2, float* rec2,
+                        const int* act, const int* nact);
 /* The boundary slots t < npb with count[t] > 0 or count2[t] > 0 (count2
  * may be null), ascending, into act[0 .. *nact) on the device; temp holds
  * boundary_targets_temp_bytes(npb) bytes of scratch. */

@@ -1235,10 +1235,10 @@ __device__ __forceinline__ void store_wall_stress(const Parameters* __restrict__
     out.xz = S.xz * inv;
     out.yz = S.yz * inv;
     store_t2(st.str, i, out);
-    if (str2) store_t2(str2, i, out);
+    store_t2(str2, i, out);
     const float rho = __ldg(&st.vel[i].w);
     store_packed_stress(nb, i, rho, out);
-    if (nb2.xs) store_packed_stress(nb2, i, rho, out);
+    store_packed_stress(nb2, i, rho, out);
 }
 
 /* ------------------------------------------------- list-driven Adami */
@@ -1246,184 +1246,131 @@ __device__ __forceinline__ void store_wall_stress(const Parameters* __restrict__
  * list of material neighbours (built with a skin; pairs at q >= 2 add
  * exact zeros, as the cell walk skips them), reading the neighbours from
  * the packed arrays (sigma_j V_j W = s_j rho_j m W with s = sigma / rho^2),
- * and writing the
- * boundary particle's new stress into the state (and into str2, the native
- * driver's other state buffer, whose boundary slots so always equal the
- * state's) and, scaled, into the packed arrays, which then need no pack of
+ * and writing the boundary particle's new stress into both state buffers
+ * and, scaled, into both stages' packed arrays, which then need no pack of
  * the boundary slots before the pair kernel.  Targets without neighbours
- * keep all of them as they were.  With `act`, thread t takes the boundary
- * slot act[t] for t < *nact (the slots whose lists can hold entries, in
- * slot order, from launch_boundary_targets): most boundary particles of a
- * wall have no material neighbour, and without the compaction a warp ran
- * as long as its longest list over lanes that had none.  Each target's
- * sums run in list order in one thread either way, so the results do not
- * depend on the compaction. */
-/* threads per block of the list-driven Adami: 128 measured against 64 and
- * 256 (256: -4 % on the 256-scenario ensemble, +10 % on the cylinder; 64:
- * +1 % and equal) */
+ * keep all of them as they were.
+ *
+ * The targets are the slots act[0 .. *nact) whose lists can hold entries
+ * (launch_boundary_targets): most boundary particles of a wall have no
+ * material neighbour.  Their number, which only the device knows, decides
+ * how many lanes share a target.  A list of about 20 entries is a chain of
+ * dependent gathers: with few targets that is the time (16 us a launch with
+ * one lane each, whatever their number), and lanes that share it divide it.
+ * With many, the lanes' idle turns and the fewer targets per warp that share
+ * a sector cost more than the chain.  So eight lanes while they come to no
+ * more than kAdamiLanes, or four to twice that, else one: 9.3 us at the 5 k
+ * column (11.3 with 4, 16 with 1), 18.2 with 4 at the 1.97 M cylinder's 70 k
+ * targets (21.0 with 8, 23.7 with 1), 44 with 1 at the 2.85 M slope (64 with
+ * 2, 88 with 8).  The launch has a lane for every boundary particle, and
+ * eight up to kAdamiLanes; blocks beyond the targets end at once (a grid of
+ * 12 blocks per SM that strides: 52 us at the slope).
+ *
+ * Lane g takes entries g, g + G, ..., U at a time: the next turn's entries
+ * are fetched ahead and a turn's gathers issued together; a pair at q >= 2
+ * and the filler of the last turn, the target's own record, get the kernel
+ * factor 0, so the loop has no branch.  From kAdamiPairTargets boundary
+ * particles on U is two instead of four (fewer filler entries: 1.17 against
+ * 1.28 ms a step at 16.2 M).  The bounds-checked build sets that threshold
+ * to 0. */
 #ifndef LQ_ADAMI_BLOCK
 #define LQ_ADAMI_BLOCK 128
 #endif
-/* Entries per group of the list-driven Adami, chosen per launch: groups of
- * four where the targets fit in about one wave of the GPU (each thread's
- * chain of dependent gathers is then the time: the cylinder's 0.34 M
- * boundary particles, ~19 entries per active one), pairs from
- * kAdamiPairTargets boundary particles on (48 registers against 62: more
- * warps and fewer filler entries where enough targets keep the memory
- * system busy; on the 256-scenario ensemble's 16.2 M, 1.17 against 1.28 ms
- * per step, groups of eight 1.24).  The sums do not depend on the group
- * size.  The bounds-checked build sets the threshold to 0, so its tests
- * take the pairs path. */
 #ifndef LQ_ADAMI_PAIR_TARGETS
 #define LQ_ADAMI_PAIR_TARGETS (4 << 20)
 #endif
 constexpr int kAdamiPairTargets = LQ_ADAMI_PAIR_TARGETS;
-/* Boundary particles below which each compacted target gets eight lanes
-: below it the gathers' latency is the time (345 k:
- * 24 us a launch with one lane, 20 with eight), above it their number
- * (1.9 M: 90 us with one lane each; not measured with eight). */
-#ifndef LQ_ADAMI_GROUP_TARGETS
-#define LQ_ADAMI_GROUP_TARGETS (1 << 20)
-#endif
-constexpr int kAdamiGroupTargets = LQ_ADAMI_GROUP_TARGETS;
-template <int kG>
-__global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(const Parameters* __restrict__ P, int npb, State st,
-                                                         const int* __restrict__ list,
-                                                         const int* __restrict__ count, int stride, NbrArrays nb,
-                                                         NbrArrays nb2, tensor2d* __restrict__ str2,
-                                                         const int* __restrict__ act,
-                                                         const int* __restrict__ nact)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npb) return;
-    if (act) {
-        /* act holds npb slots, so both loads are issued together */
-        const int na = __ldg(nact), a = __ldg(act + i);
-        if (i >= na) return;
-        i = a;
-    }
-    const int n = min(__ldg(count + i), LQ_NBR_CAP);
-    if (n == 0) return;
-    const int np_all = __ldg(&P->np);
-    const float ih = __ldg(&P->i_h), m = __ldg(&P->m), Cw = __ldg(&P->kernel_normalization_par);
-    const float4 xi = __ldg(st.pos + i);
-    tensor2d S = make_tensor2d(0.0f);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    /* groups of kG entries, the next group's entries fetched ahead and
-     * every gather of a group issued together; a pair at q >= 2 (and the
-     * filler of the last group, the target's own record) gets the kernel
-     * factor 0 and adds exact zeros, so the loop has no branch and its sums
-     * do not depend on kG */
-    const int* p = list + i;
-    int nxt[kG];
-#pragma unroll
-    for (int u = 0; u < kG; ++u) nxt[u] = u < n ? __ldg(p + (size_t)u * stride) : i;
-    for (int k = 0; k < n; k += kG) {
-        int j[kG];
-#pragma unroll
-        for (int u = 0; u < kG; ++u) {
-            j[u] = lq_in_range(nxt[u], np_all) ? nxt[u] : i;
-            nxt[u] = k + kG + u < n ? __ldg(p + (size_t)(k + kG + u) * stride) : i;
-        }
-        float4 xr[kG], sa[kG];
-        float2 sb[kG];
-#pragma unroll
-        for (int u = 0; u < kG; ++u) {
-            load_xs(nb, j[u], xr[u], sa[u]);
-            sb[u] = __ldg(reinterpret_cast<const float2*>(nb.sb + j[u]));
-        }
-#pragma unroll
-        for (int u = 0; u < kG; ++u) {
-            const float3 d = make_float3(xi.x - xr[u].x, xi.y - xr[u].y, xi.z - xr[u].z);
-            /* the approximate square root and quotient of the pair kernel */
-            const float q = sqrt_approx(d.x * d.x + d.y * d.y + d.z * d.z) * ih;
-            const float t = k + u < n ? fmaxf(2.0f - q, 0.0f) : 0.0f;
-            const float ker = Cw * t * t * t * t * (q + 0.5f);
-            const float kv = ker * __fdividef(m, xr[u].w);
-            const float cs = m * xr[u].w * ker;
-            S.xx += sa[u].x * cs;
-            S.yy += sa[u].y * cs;
-            S.zz += sa[u].z * cs;
-            S.xy += sa[u].w * cs;
-            S.xz += sb[u].x * cs;
-            S.yz += sb[u].y * cs;
-            acc.x += d.x * kv;
-            acc.y += d.y * kv;
-            acc.z += d.z * kv;
-            acc.w += kv;
-        }
-    }
-    if (acc.w > 0.0f) store_wall_stress(P, st, i, S, acc, str2, nb, nb2);
-}
+constexpr int kAdamiLanes = 1 << 18;
 
-/* The list-driven Adami with G lanes per target, for the sizes at which
- * k_adami_packed's chain of dependent gathers is the time (16 us a launch
- * from 5 k to 1 M particles; 9.5 so, 17 at the 1.97 M cylinder): lane g
- * takes entries g, g + G, ..., two at a time, and the ten sums are combined
- * with shuffles.  A fixed grid walks the compacted targets, whose number
- * only the device knows. */
-template <int G>
-__global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_group(const Parameters* __restrict__ P, State st,
-                                                                const int* __restrict__ list,
-                                                                const int* __restrict__ count, int stride,
-                                                                NbrArrays nb, NbrArrays nb2,
-                                                                tensor2d* __restrict__ str2,
-                                                                const int* __restrict__ act,
-                                                                const int* __restrict__ nact)
+struct WallSums {
+    const Parameters* P;
+    State st;
+    const int* list;
+    const int* count;
+    int stride;
+    NbrArrays nb, nb2;
+    tensor2d* str2;
+    const int* act;
+};
+
+template <int G, int U>
+__device__ __forceinline__ void adami_targets(const WallSums& w, int na)
 {
     const int g = threadIdx.x % G;
     const unsigned mates = (unsigned)((1ull << G) - 1ull) << (threadIdx.x & 31 & ~(G - 1));
-    const int step = gridDim.x * (LQ_ADAMI_BLOCK / G), na = __ldg(nact);
-    const int np_all = __ldg(&P->np);
-    const float ih = __ldg(&P->i_h), m = __ldg(&P->m), Cw = __ldg(&P->kernel_normalization_par);
+    const int step = gridDim.x * (LQ_ADAMI_BLOCK / G);
+    const int np_all = __ldg(&w.P->np);
+    const float ih = __ldg(&w.P->i_h), m = __ldg(&w.P->m), Cw = __ldg(&w.P->kernel_normalization_par);
     for (int a = (blockIdx.x * LQ_ADAMI_BLOCK + threadIdx.x) / G; a < na; a += step) {
-        const int i = __ldg(act + a);
-        const int n = min(__ldg(count + i), LQ_NBR_CAP);
-        const float4 xi = __ldg(st.pos + i);
-        float sum[10] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const int* p = list + i;
-        for (int k = g; k < n; k += 2 * G) {
-            int j[2];
-            float4 xr[2], sa[2];
-            float2 sb[2];
+        const int i = __ldg(w.act + a);
+        const int n = min(__ldg(w.count + i), LQ_NBR_CAP);
+        const float4 xi = __ldg(w.st.pos + i);
+        tensor2d S = make_tensor2d(0.0f);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto entry = [&](int k) {
+            const int j = k < n ? __ldg(w.list + (size_t)k * w.stride + i) : i;
+            return lq_in_range(j, np_all) ? j : i;
+        };
+        int nxt[U];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                j[u] = k + u * G < n ? __ldg(p + (size_t)(k + u * G) * stride) : i;
-                if (!lq_in_range(j[u], np_all)) j[u] = i;
+        for (int u = 0; u < U; ++u) nxt[u] = entry(g + u * G);
+        for (int k = g; k < n; k += U * G) {
+            int j[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                j[u] = nxt[u];
+                nxt[u] = entry(k + (U + u) * G);
+            }
+            float4 xr[U], sa[U];
+            float2 sb[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                load_xs(w.nb, j[u], xr[u], sa[u]);
+                sb[u] = __ldg(reinterpret_cast<const float2*>(w.nb.sb + j[u]));
             }
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                load_xs(nb, j[u], xr[u], sa[u]);
-                sb[u] = __ldg(reinterpret_cast<const float2*>(nb.sb + j[u]));
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const float dx = xi.x - xr[u].x, dy = xi.y - xr[u].y, dz = xi.z - xr[u].z;
+                /* the approximate square root and quotient of the pair kernel */
                 const float q = sqrt_approx(dx * dx + dy * dy + dz * dz) * ih;
                 const float t = k + u * G < n ? fmaxf(2.0f - q, 0.0f) : 0.0f;
                 const float ker = Cw * t * t * t * t * (q + 0.5f);
                 const float kv = ker * __fdividef(m, xr[u].w);
                 const float cs = m * xr[u].w * ker;
-                sum[0] += sa[u].x * cs;
-                sum[1] += sa[u].y * cs;
-                sum[2] += sa[u].z * cs;
-                sum[3] += sa[u].w * cs;
-                sum[4] += sb[u].x * cs;
-                sum[5] += sb[u].y * cs;
-                sum[6] += dx * kv;
-                sum[7] += dy * kv;
-                sum[8] += dz * kv;
-                sum[9] += kv;
+                S.xx += sa[u].x * cs;
+                S.yy += sa[u].y * cs;
+                S.zz += sa[u].z * cs;
+                S.xy += sa[u].w * cs;
+                S.xz += sb[u].x * cs;
+                S.yz += sb[u].y * cs;
+                acc.x += dx * kv;
+                acc.y += dy * kv;
+                acc.z += dz * kv;
+                acc.w += kv;
             }
         }
+        if (G > 1) {
+            float* v[10] = {&S.xx, &S.yy, &S.zz, &S.xy, &S.xz, &S.yz, &acc.x, &acc.y, &acc.z, &acc.w};
 #pragma unroll
-        for (int k = 0; k < 10; ++k)
+            for (int k = 0; k < 10; ++k)
 #pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(mates, sum[k], o, G);
-        if (g == 0 && sum[9] > 0.0f)
-            store_wall_stress(P, st, i, make_tensor2d(sum[0], sum[1], sum[2], sum[3], sum[4], sum[5]),
-                              make_float4(sum[6], sum[7], sum[8], sum[9]), str2, nb, nb2);
+                for (int o = G / 2; o > 0; o >>= 1) *v[k] += __shfl_xor_sync(mates, *v[k], o, G);
+        }
+        if (g == 0 && acc.w > 0.0f) store_wall_stress(w.P, w.st, i, S, acc, w.str2, w.nb, w.nb2);
     }
+}
+
+__global__ void __launch_bounds__(LQ_ADAMI_BLOCK) k_adami_packed(WallSums w, const int* __restrict__ nact, bool pairs)
+{
+    const int na = __ldg(nact);
+    if (pairs)
+        adami_targets<1, 2>(w, na);
+    else if (na <= kAdamiLanes / 8)
+        adami_targets<8, 2>(w, na);
+    else if (na <= kAdamiLanes / 2)
+        adami_targets<4, 2>(w, na);
+    else
+        adami_targets<1, 4>(w, na);
 }
 
 /* ------------------------------------------ list-driven Shepard filters */
@@ -1754,24 +1701,15 @@ int launch_adami_packed(const Parameters* ph, const Parameters* pd, const State&
                         float* rec, cudaStream_t s, tensor2d* str2, float* rec2, const int* act, const int* nact)
 {
     if (ph->npb <= 0) return LQ_OK;
-    if (!act != !nact) return set_error(LQ_ERR_ARG, "Adami: compacted targets need both act and nact");
+    if (!act || !nact || !str2 || !rec2)
+        return set_error(LQ_ERR_ARG, "Adami: the compacted targets and both stages' buffers are required");
     if (nl.stride < ph->npb) return set_error(LQ_ERR_ARG, "Adami: list stride %d < %d targets", nl.stride, ph->npb);
-    const NbrArrays nb = nbr_arrays(rec, ph->np);
-    const NbrArrays nb2 = rec2 ? nbr_arrays(rec2, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
-    const int grid = blocks_for(ph->npb, LQ_ADAMI_BLOCK);
-    if (act && ph->npb < kAdamiGroupTargets) {
-        int dev = 0, sms = 0;
-        LQ_TRY_CUDA(cudaGetDevice(&dev), "Adami");
-        LQ_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "Adami");
-        const int all = blocks_for((long long)ph->npb * 8, LQ_ADAMI_BLOCK), most = sms * 12;
-        k_adami_group<8><<<all < most ? all : most, LQ_ADAMI_BLOCK, 0, s>>>(pd, st, nl.list, nl.count, nl.stride, nb,
-                                                                            nb2, str2, act, nact);
-    } else if (ph->npb >= kAdamiPairTargets)
-        k_adami_packed<2><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, nb2, str2, act,
-                                                          nact);
-    else
-        k_adami_packed<4><<<grid, LQ_ADAMI_BLOCK, 0, s>>>(pd, ph->npb, st, nl.list, nl.count, nl.stride, nb, nb2, str2, act,
-                                                          nact);
+    const bool pairs = ph->npb >= kAdamiPairTargets;
+    const long long eight = ph->npb * 8ll, few = eight < kAdamiLanes ? eight : kAdamiLanes;
+    const long long lanes = ph->npb > few ? ph->npb : few;
+    const int grid = blocks_for(lanes, LQ_ADAMI_BLOCK);
+    const WallSums w{pd, st, nl.list, nl.count, nl.stride, nbr_arrays(rec, ph->np), nbr_arrays(rec2, ph->np), str2, act};
+    k_adami_packed<<<grid, LQ_ADAMI_BLOCK, 0, s>>>(w, nact, pairs);
     LQ_TRY_CUDA(cudaGetLastError(), "k_adami_packed");
     return LQ_OK;
 }
