@@ -145,8 +145,8 @@ int identity_reset(const int* key, int np);
 void identity_release(const int* key);
 bool identity_find(const int* key, GridIdentity* out);
 
-int gather_float4(int n, const int* idx, const float4* in, float4* out, cudaStream_t s);
-int gather_tensor2d(int n, const int* idx, const tensor2d* in, tensor2d* out, cudaStream_t s);
+int sort_float4(int n, const int* idx, float4* data, float4* cache, cudaStream_t s);
+int sort_tensor2d(int n, const int* idx, tensor2d* data, tensor2d* cache, cudaStream_t s);
 /* Gathers all five state arrays in one pass: out[i] = in[idx[i]]. */
 int gather_state(int n, const int* idx, const State& in, const State& out, cudaStream_t s);
 
