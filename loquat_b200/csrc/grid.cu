@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kBlock) k_scatter(int np, const int* __restric
 
 /* What a search writes of its order besides part_idx: the sorted keys, the
  * per-cell bounds and the identities of the slots' particles (each may be
- * null; ident_out[slot] = ident_in[previous slot]). */
+ * null; ident_out[slot] = ident_in[previous slot], or the previous slot
+ * itself without ident_in: identities that start here). */
 struct OrderOutputs {
     int* part_cel;
     int* beg;
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, int np, const 
     }
     auto place = [&](int d, int v, int cell) {      /* slot d holds previous slot v's particle */
         if (out.part_cel) out.part_cel[d] = cell;
-        if (out.ident_out) out.ident_out[d] = lq_in_range(v, np) ? __ldg(out.ident_in + v) : -1;
+        if (out.ident_out) out.ident_out[d] = !lq_in_range(v, np) ? -1 : out.ident_in ? __ldg(out.ident_in + v) : v;
     };
     unsigned todo = __ballot_sync(FULL, n > 0);
     int k = __ffs((int)todo) - 1;
@@ -292,11 +293,16 @@ int scan_scratch_bytes(int ncell, size_t* bytes)
 /* --------------------------------------------- identities of the grids */
 namespace {
 
+/* `started`: ident holds the identity of each of np slots.  Not so before
+ * a grid's first search, nor after a search over another particle count,
+ * which does not follow the other slots' particles: the next search over np
+ * particles then starts them again, on its own stream. */
 struct IdentityRecord {
     int* ident = nullptr;
     int* tmp = nullptr;
     int np = 0;
     long long gen = 0;
+    bool started = false;
 };
 std::mutex g_id_mu;
 std::unordered_map<const int*, IdentityRecord> g_ids;
@@ -309,12 +315,10 @@ IdentityRecord* identity_for_search(const int* key, int np)
     auto it = g_ids.find(key);
     if (it == g_ids.end()) return nullptr;
     IdentityRecord& r = it->second;
-    if (np != r.np) {
-        /* a search over another particle count: identities restart */
-        r.gen = ++g_id_gen;
-        if (np > r.np) return nullptr;
-    }
-    return np > 0 ? &r : nullptr;
+    if (np == r.np) return np > 0 ? &r : nullptr;
+    r.started = false;
+    r.gen = ++g_id_gen;
+    return nullptr;
 }
 
 }  // namespace
@@ -351,7 +355,7 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
             id = identity_for_search(identity_key, np);
         }
         if (id) {
-            out.ident_in = id->ident;
+            out.ident_in = id->started ? id->ident : nullptr;
             out.ident_out = id->tmp;
         }
         /* few cells: fewer per warp, whose chain of cells is the time
@@ -362,7 +366,10 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
         else
             k_cell_order<16><<<blocks_for(ncell, kBlock / 2), kBlock, 0, s>>>(ncell, np, g.start, g.part_idx, out);
         LQ_TRY_CUDA(cudaGetLastError(), "k_cell_order");
-        if (id) std::swap(id->ident, id->tmp);
+        if (id) {
+            std::swap(id->ident, id->tmp);
+            id->started = true;
+        }
     }
     return LQ_OK;
 }
@@ -411,16 +418,6 @@ int bounds_count_grid(unsigned long long* v)
     return LQ_OK;
 }
 
-namespace {
-
-__global__ void __launch_bounds__(kBlock) k_iota(int n, int* __restrict__ p)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = i;
-}
-
-}  // namespace
-
 int identity_reset(const int* key, int np)
 {
     std::lock_guard<std::mutex> lock(g_id_mu);
@@ -441,10 +438,7 @@ int identity_reset(const int* key, int np)
         r.np = np;
     }
     r.gen = ++g_id_gen;
-    if (np > 0) {
-        k_iota<<<blocks_for(np), kBlock>>>(np, r.ident);
-        LQ_TRY_CUDA(cudaGetLastError(), "k_iota");
-    }
+    r.started = false;      /* the first search starts the identities */
     return LQ_OK;
 }
 
@@ -462,7 +456,7 @@ bool identity_find(const int* key, GridIdentity* out)
 {
     std::lock_guard<std::mutex> lock(g_id_mu);
     auto it = g_ids.find(key);
-    if (it == g_ids.end() || !it->second.ident) return false;
+    if (it == g_ids.end() || !it->second.started) return false;
     out->ident = it->second.ident;
     out->np = it->second.np;
     out->gen = it->second.gen;

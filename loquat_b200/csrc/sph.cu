@@ -2030,10 +2030,10 @@ __global__ void __launch_bounds__(256) k_moved_half_skin(int np, const float4* _
 
 /* What a call does per slot besides its lists: a build (*moved, or moved
  * null) is recorded, each particle's build slot and position by identity;
- * the particle's neighbour record is packed at its build slot (not for a
- * particle that has none); and each material target gets its list's row,
- * that slot less npb (-1: no carried list, the pair kernel walks its
- * stencil).  One thread counts the decision. */
+ * the particle's neighbour record is packed at its build slot, which in a
+ * build is the slot itself (not for a particle that has none); and each
+ * material target gets its list's row, that slot less npb (-1: no carried
+ * list, the pair kernel walks its stencil).  One thread counts the decision. */
 __global__ void __launch_bounds__(256) k_carry(int np, int npb, lqb::State st, const int* __restrict__ ident,
                                                const int* __restrict__ moved, float4* __restrict__ xbuild,
                                                int* __restrict__ build_of, lqb::NbrArrays nb, int* __restrict__ rows,
@@ -2045,11 +2045,11 @@ __global__ void __launch_bounds__(256) k_carry(int np, int npb, lqb::State st, c
     if (c == 0) tally[build ? 0 : 1] += 1;
     const int id = __ldg(ident + c);
     const float4 x = __ldg(st.pos + c);
-    int o = -1;
+    int o = build ? c : -1;     /* a build's lists name its own slots, every one of them */
     if ((unsigned)id < (unsigned)np) {
         if (build) {
             xbuild[id] = x;
-            build_of[id] = o = c;
+            build_of[id] = c;
         } else {
             o = build_of[id];
             if ((unsigned)o >= (unsigned)np) o = -1;
