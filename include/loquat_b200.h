@@ -114,7 +114,8 @@ int lq_interaction_reserve(const void* par_host);
  * the cell_beg passed belongs to a grid of this library (lq_grid_* or the
  * drop-in LoquatGrid), whose searches track each particle's identity,
  * the caller has re-sorted its arrays after each search (as the reference
- * does), and no particle has moved half a skin of 0.05 h since the build;
+ * does), the Parameters have the h and the cell counts of the build, and
+ * no particle has moved half a skin of 0.05 h since the build;
  * the grid's searches and the interaction must run on one stream. */
 int lq_interaction_stats(long long* rebuilds, long long* reuses);
 

@@ -1924,6 +1924,8 @@ struct DropInWorkspace {
     const int* key = nullptr;       /* the grid (its cell_beg) the carried lists belong to */
     long long gen = -1;
     int np_built = 0, npb_built = 0;
+    float h_built = 0.0f;           /* what the lists hold depends on the cut-off and on the cells walked */
+    int cells_built[3] = {0, 0, 0};
     bool built = false;
     long long rebuilds = 0, reuses = 0;   /* counts of earlier workspaces (tally holds this one's) */
     std::vector<void*> allocs;
@@ -2126,8 +2128,9 @@ extern "C" int lq_particle_interaction(const void* par_host, const void* par_dev
          * The device decides (no host synchronisation): the list build is
          * enqueued and returns at once when it is not taken. */
         const float skin = kDropInSkinOverH * ph->h;
-        const bool carried =
-            w->built && w->key == cell_beg && w->gen == gi.gen && w->np_built == np && w->npb_built == npb;
+        const bool carried = w->built && w->key == cell_beg && w->gen == gi.gen && w->np_built == np &&
+                             w->npb_built == npb && w->h_built == ph->h && w->cells_built[0] == ph->cell_num_x &&
+                             w->cells_built[1] == ph->cell_num_y && w->cells_built[2] == ph->cell_num_z;
         const int* moved = nullptr;
         if (carried) {
             LQ_TRY_CUDA(cudaMemsetAsync(w->moved, 0, sizeof(int), s), "moved flag");
@@ -2150,6 +2153,10 @@ extern "C" int lq_particle_interaction(const void* par_host, const void* par_dev
         w->gen = gi.gen;
         w->np_built = np;
         w->npb_built = npb;
+        w->h_built = ph->h;
+        w->cells_built[0] = ph->cell_num_x;
+        w->cells_built[1] = ph->cell_num_y;
+        w->cells_built[2] = ph->cell_num_z;
         return lqb::launch_interaction_list(ph, pd, st, r, c, w->nl, s, lqb::Frames(), false, w->rec, kDropInShape,
                                             false, nullptr, w->rows);
     }
