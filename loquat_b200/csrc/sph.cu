@@ -1979,7 +1979,9 @@ int size_workspace(DropInWorkspace& w, const Parameters* ph)
     A((void**)&n.moved, sizeof(int));
     A((void**)&n.tally, 2 * sizeof(int));
     if (st == LQ_OK) {
-        const cudaError_t e = cudaMemset(n.tally, 0, 2 * sizeof(int));
+        /* done before any stream's call can count */
+        cudaError_t e = cudaMemset(n.tally, 0, 2 * sizeof(int));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
         if (e != cudaSuccess) st = lqb::set_error(LQ_ERR_CUDA, "interaction workspace: %s", cudaGetErrorString(e));
     }
     if (st != LQ_OK) {
