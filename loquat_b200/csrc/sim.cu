@@ -662,6 +662,16 @@ int upload(LqSim* S, const float* pos, const float* vel, const float* idep, cons
     return LQ_OK;
 }
 
+/* A caller's table into device memory, there when the call returns: ordered
+ * on the simulation's own stream, which the default stream does not hold up
+ * (a plain copy from pageable memory may return before it has arrived). */
+int upload_table(LqSim* S, void* dst, const void* src, size_t bytes, const char* what)
+{
+    LQ_TRY_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, S->stream), what);
+    LQ_TRY_CUDA(cudaStreamSynchronize(S->stream), what);
+    return LQ_OK;
+}
+
 int set_flag(LqSim* S, int v) { return lqb::fill_int(S->rebuild, 1, v, S->stream); }
 
 /* New positions, order or list settings: sort and build all lists first. */
@@ -982,7 +992,7 @@ extern "C" int lq_sim_set_materials(void* sim, int n, const float* table)
     float* d = nullptr;
     if (n > 0) {
         LQ_TRY(dev_alloc(S, (void**)&d, sizeof(float) * 5 * (size_t)n));
-        LQ_TRY_CUDA(cudaMemcpy(d, table, sizeof(float) * 5 * (size_t)n, cudaMemcpyHostToDevice), "material table");
+        LQ_TRY(upload_table(S, d, table, sizeof(float) * 5 * (size_t)n, "material table"));
     }
     S->mt.p = d;
     S->mt.n = n;
@@ -1009,7 +1019,7 @@ extern "C" int lq_sim_set_hypoplastic(void* sim, int n, const float* table)
     LQ_TRY_CUDA(cudaStreamSynchronize(S->stream), "set hypoplastic");
     float* d = nullptr;
     LQ_TRY(dev_alloc(S, (void**)&d, sizeof(float) * 10 * (size_t)n));
-    LQ_TRY_CUDA(cudaMemcpy(d, table, sizeof(float) * 10 * (size_t)n, cudaMemcpyHostToDevice), "hypoplastic table");
+    LQ_TRY(upload_table(S, d, table, sizeof(float) * 10 * (size_t)n, "hypoplastic table"));
     void* derived = nullptr;
     LQ_TRY(dev_alloc(S, &derived, lqb::vw_row_bytes() * (size_t)n));
     if (!S->subq.item) {
@@ -1040,7 +1050,7 @@ extern "C" int lq_sim_set_frames(void* sim, int n, const int* rows)
     int* d = nullptr;
     if (n > 0) {
         LQ_TRY(dev_alloc(S, (void**)&d, sizeof(int) * 2 * (size_t)n));
-        LQ_TRY_CUDA(cudaMemcpy(d, rows, sizeof(int) * 2 * (size_t)n, cudaMemcpyHostToDevice), "frame table");
+        LQ_TRY(upload_table(S, d, rows, sizeof(int) * 2 * (size_t)n, "frame table"));
     }
     S->fr.rows = d;
     S->fr.n = n;
