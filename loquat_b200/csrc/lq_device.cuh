@@ -105,15 +105,17 @@ __device__ __forceinline__ bool zrun_range(const Cells& c, int base, int zlo, in
         e = __ldg(c.start + base + zhi + 1);
         return e > s;
     }
-    s = -1;
+    /* a caller's bounds: an empty cell has beg -1, or beg and end alike */
+    s = e = -1;
     for (int z = zlo; z <= zhi; ++z) {
-        int b = __ldg(c.beg + base + z);
-        if (b != -1) {
-            if (s < 0) s = b;
-            e = __ldg(c.end + base + z);
-        }
+        const int b = __ldg(c.beg + base + z);
+        if (b == -1) continue;
+        const int f = __ldg(c.end + base + z);
+        if (f <= b) continue;
+        if (s < 0) s = b;
+        e = f;
     }
-    return s >= 0;
+    return e > s;
 }
 
 /* Jaumann co-rotational term with spin (W_yx, W_zx, W_zy)

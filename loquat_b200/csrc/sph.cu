@@ -1135,18 +1135,22 @@ __device__ __forceinline__ CellSums sum_material_cells(const Parameters* __restr
         bool apart = false;
         if (col < 9 && X >= 0 && X < nx && Y >= 0 && Y < ny) {
             const int cell = L + (X * ny + Y) * nz + zlo;
-            int b[3];
-#pragma unroll
-            for (int z = 0; z < 3; ++z) b[z] = zlo + z <= zhi ? __ldg(cells.beg + cell + z) : -1;
+            int b[3], f[3];
 #pragma unroll
             for (int z = 0; z < 3; ++z) {
-                if (b[z] == -1) continue;
+                const bool in = zlo + z <= zhi;
+                b[z] = in ? __ldg(cells.beg + cell + z) : -1;
+                f[z] = in ? __ldg(cells.end + cell + z) : -1;
+            }
+#pragma unroll
+            for (int z = 0; z < 3; ++z) {
+                if (b[z] == -1 || f[z] <= b[z]) continue;   /* empty, by either mark */
                 if (e == 0) {
                     s = b[z];
                 } else if (b[z] != e) {
                     apart = true;
                 }
-                e = __ldg(cells.end + cell + z);
+                e = f[z];
             }
         }
         const bool any_apart = __any_sync(FULL, apart);
