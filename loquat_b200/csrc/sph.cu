@@ -24,6 +24,7 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include "lq_internal.cuh"
+#include "lq_lanes.h"
 #include "lq_tile.h"
 #include "lq_device.cuh"
 #include "lq_integrate.cuh"
@@ -1187,7 +1188,7 @@ __device__ __forceinline__ CellSums sum_material_cells(const Parameters* __restr
 __global__ void __launch_bounds__(kBlock) k_adami(const Parameters* __restrict__ P, int npb, State st, Cells cells)
 {
     __shared__ int queue[kBlock / kCellLanes][kCellQueue];
-    const int i = (blockIdx.x * kBlock + threadIdx.x) / kCellLanes;
+    const int i = lane_target(blockIdx.x, threadIdx.x, kBlock, kCellLanes);
     const bool active = i < npb;
     const float4 xi = active ? __ldg(st.pos + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     const CellSums r = sum_material_cells(P, st, cells, active, xi, queue[threadIdx.x / kCellLanes]);
@@ -1210,7 +1211,7 @@ __global__ void __launch_bounds__(kBlock) k_shepard(const Parameters* __restrict
                                                     tensor2d* __restrict__ out_str, Cells cells)
 {
     __shared__ int queue[kBlock / kCellLanes][kCellQueue];
-    const int i = npb + (blockIdx.x * kBlock + threadIdx.x) / kCellLanes;
+    const int i = npb + lane_target(blockIdx.x, threadIdx.x, kBlock, kCellLanes);
     const bool active = i < np;
     const float4 xi = active ? __ldg(st.pos + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     CellSums r = sum_material_cells(P, st, cells, active, xi, queue[threadIdx.x / kCellLanes]);
