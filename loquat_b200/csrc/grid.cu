@@ -205,47 +205,82 @@ __device__ __forceinline__ tensor2d element(const tensor2d* p, int i) { return l
 __device__ __forceinline__ void put(float4* p, int i, const float4& v) { p[i] = v; }
 __device__ __forceinline__ void put(tensor2d* p, int i, const tensor2d& v) { store_t2(p, i, v); }
 
-/* One array permuted in place through its cache: the elements gathered into
- * the cache and, when every block has done so (kBack; a cooperative launch),
- * copied back, where the cache is still in L2.  A gather and a device copy
- * of its own, two launches whose ends the GPU waits for, took 11 us a call
- * for 4 k to 53 k elements instead of 5.6, and for 1.03 M 14.9 instead of
- * 10.5 (float4) and 17.7 instead of 15.3 (tensor2d); above that the memory
- * bounds it: 20.5 and 38.2 at 2.3 M (27 and 46), 74 and 114 at 6.6 M (86
- * and 118).  Four blocks per SM leave each thread registers for its gathers
- * (six: 11.7 and 18.0 at 1.03 M). */
-constexpr int kSortBlocks = 4;
-template <bool kBack, class T>
-__global__ void __launch_bounds__(kBlock, kSortBlocks) k_sort_array(int n, const int* __restrict__ idx, T* data, T* cache)
+/* One array permuted in place through its cache: gathered into the cache,
+ * then copied back, where the cache is still in L2.  Each thread takes
+ * kSortItems elements, a block's apart by its threads, with all loads issued
+ * before the first store.
+ *
+ * Two plain launches: a sort goes on beside another stream's sorts and
+ * beside a resident kernel of the caller's, where a cooperative launch
+ * with a grid barrier waits until all its blocks fit on the device at once.
+ * The copy is launched while the gather runs (its blocks come onto the
+ * device once every block of the gather has, and then wait for the gather's
+ * end), which takes the gap between the two out: 3.3 us a call in a graph
+ * for 11 k to 150 k float4 elements, 16.2 for 2.3 M and 69 for 6.6 M
+ * (tensor2d 35 and 104), where the cooperative launch took 3.7 to 5.1, 18.7
+ * and 73 (37 and 112); called one by one 6.4 us against 6.1 below 150 k. */
+constexpr int kSortItems = 4;
+
+template <class T>
+__device__ __forceinline__ void gather_items(int n, long long first, const int* idx, const T* data, T* cache)
 {
-    const int t = blockIdx.x * kBlock + threadIdx.x, all = gridDim.x * kBlock;
-    for (long long at = t; at < n; at += 4ll * all) {
-        int j[4];
-        T v[4];
+    int j[kSortItems];
+    T v[kSortItems];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) j[u] = at + (long long)u * all < n ? __ldg(idx + at + (long long)u * all) : -1;
+    for (int u = 0; u < kSortItems; ++u) j[u] = first + u * kBlock < n ? __ldg(idx + first + u * kBlock) : -1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (j[u] >= 0 && lq_in_range(j[u], n)) v[u] = element(data, j[u]);
+    for (int u = 0; u < kSortItems; ++u)
+        if (j[u] >= 0 && lq_in_range(j[u], n)) v[u] = element(data, j[u]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (j[u] >= 0 && lq_in_range(j[u], n)) put(cache, (int)(at + (long long)u * all), v[u]);
-    }
-    if (!kBack) return;
-    cooperative_groups::this_grid().sync();
-    constexpr int kWords = sizeof(T) / sizeof(float2);
-    const float2* from = reinterpret_cast<const float2*>(cache);
-    float2* to = reinterpret_cast<float2*>(data);
-    const long long words = (long long)n * kWords;
-    for (long long at = t; at < words; at += 8ll * all) {
-        float2 v[8];
+    for (int u = 0; u < kSortItems; ++u)
+        if (j[u] >= 0 && lq_in_range(j[u], n)) put(cache, (int)(first + u * kBlock), v[u]);
+}
+
+template <class W>
+__device__ __forceinline__ void copy_items(long long words, long long first, const W* from, W* to)
+{
+    W v[kSortItems];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (at + (long long)u * all < words) v[u] = from[at + (long long)u * all];
+    for (int u = 0; u < kSortItems; ++u)
+        if (first + u * kBlock < words) v[u] = from[first + u * kBlock];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (at + (long long)u * all < words) to[at + (long long)u * all] = v[u];
-    }
+    for (int u = 0; u < kSortItems; ++u)
+        if (first + u * kBlock < words) to[first + u * kBlock] = v[u];
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_sort_gather(int n, const int* __restrict__ idx, const T* data, T* cache)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    gather_items(n, (long long)blockIdx.x * (kSortItems * kBlock) + threadIdx.x, idx, data, cache);
+}
+
+template <class W>
+__global__ void __launch_bounds__(kBlock) k_sort_copy_back(long long words, const W* from, W* to)
+{
+    cudaGridDependencySynchronize();
+    copy_items(words, (long long)blockIdx.x * (kSortItems * kBlock) + threadIdx.x, from, to);
+}
+
+/* Few elements: both steps by one cluster of blocks in one launch, which
+ * needs room for eight blocks in one part of the device only.  Up to the
+ * elements that its threads take at once: 2.9 us a call in a graph for 4.5 k
+ * float4 elements and 3.8 for tensor2d (3.0 and 3.3 with two launches), but
+ * 5.7 us called one by one instead of 9.7, since a caller with so few
+ * elements waits for the host; for 11 k tensor2d elements 5.7 us, 3.8 with two
+ * launches. */
+constexpr int kSortCluster = 8;
+constexpr int kSortSmall = kSortCluster * kSortItems * kBlock;
+template <class W, class T>
+__global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kBlock)
+    k_sort_small(int n, const int* __restrict__ idx, T* data, T* cache)
+{
+    const int first = blockIdx.x * (kSortItems * kBlock) + threadIdx.x;
+    gather_items(n, first, idx, data, cache);
+    cooperative_groups::this_cluster().sync();
+    const int words = n * (int)(sizeof(T) / sizeof(W));
+    for (int at = first; at < words; at += kSortSmall)
+        copy_items(words, at, reinterpret_cast<const W*>(cache), reinterpret_cast<W*>(data));
 }
 
 __global__ void __launch_bounds__(kBlock) k_gather_state(int n, const int* __restrict__ idx, State in, State out)
@@ -374,36 +409,41 @@ int grid_search(const Parameters* ph, const Parameters* pd, const float4* pos, G
     return LQ_OK;
 }
 
-template <class T>
+template <class W, class T>
 static int sort_array(int n, const int* idx, T* data, T* cache, cudaStream_t s)
 {
     if (n <= 0) return LQ_OK;
-    int dev = 0, sms = 0;
-    LQ_TRY_CUDA(cudaGetDevice(&dev), "k_sort_array");
-    LQ_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "k_sort_array");
-    const int need = blocks_for(n), most = sms * kSortBlocks;
-    void* args[] = {&n, &idx, &data, &cache};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sort_array<true, T>, need < most ? need : most,
-                                                      kBlock, args, 0, s);
-    if (e != cudaErrorCooperativeLaunchTooLarge) {
-        LQ_TRY_CUDA(e, "k_sort_array");
+    if (n <= kSortSmall) {
+        k_sort_small<W><<<kSortCluster, kBlock, 0, s>>>(n, idx, data, cache);
+        LQ_TRY_CUDA(cudaGetLastError(), "k_sort_small");
         return LQ_OK;
     }
-    cudaGetLastError();     /* the process has a part of the device only: in two launches */
-    k_sort_array<false, T><<<blocks_for(n, 4 * kBlock), kBlock, 0, s>>>(n, idx, data, cache);
-    LQ_TRY_CUDA(cudaGetLastError(), "k_sort_array");
-    LQ_TRY_CUDA(cudaMemcpyAsync(data, cache, sizeof(T) * (size_t)n, cudaMemcpyDeviceToDevice, s), "copy back");
+    k_sort_gather<<<blocks_for(n, kSortItems * kBlock), kBlock, 0, s>>>(n, idx, data, cache);
+    LQ_TRY_CUDA(cudaGetLastError(), "k_sort_gather");
+    const long long words = (long long)n * (int)(sizeof(T) / sizeof(W));
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks_for(words, kSortItems * kBlock));
+    c.blockDim = dim3(kBlock);
+    c.stream = s;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    LQ_TRY_CUDA(cudaLaunchKernelEx(&c, k_sort_copy_back<W>, words, reinterpret_cast<const W*>(cache),
+                                   reinterpret_cast<W*>(data)),
+                "k_sort_copy_back");
     return LQ_OK;
 }
 
 int sort_float4(int n, const int* idx, float4* data, float4* cache, cudaStream_t s)
 {
-    return sort_array(n, idx, data, cache, s);
+    return sort_array<float4>(n, idx, data, cache, s);
 }
 
 int sort_tensor2d(int n, const int* idx, tensor2d* data, tensor2d* cache, cudaStream_t s)
 {
-    return sort_array(n, idx, data, cache, s);
+    return sort_array<float2>(n, idx, data, cache, s);
 }
 
 /* This translation unit's count of bounds violations (always 0 without
