@@ -88,7 +88,7 @@ struct LqSim {
     lqb::MaterialTable vw;             /* von Wolffersdorff rows (model 3) */
     lqb::SubstepQueue subq;            /* particles with more than one sub-step (model 3) */
     float* rec = nullptr;              /* packed neighbour data of S, np x 13 floats */
-    float* rec2 = nullptr;             /* and of the stage buffer S2 */
+    float* rec2 = nullptr;             /* and of the stage buffer S2, in T's memory (alloc_scratch_state) */
     float* rho_f = nullptr;            /* density filter output (LQ_SIM_DENSITY_FILTER) */
     int pair_shape = 0;                /* launch shape of the pair kernel (lqb::kPairShapes) */
     lqb::TileOrder tile;               /* targets in tile order (tiled shapes; allocated on first use) */
@@ -171,6 +171,27 @@ int alloc_state(LqSim* S, State& st, float4* idep = nullptr)
     if (S->flags & LQ_SIM_MIXED) {
         LQ_TRY(dev_alloc(S, (void**)&st.xlo, n * sizeof(float4)));
         LQ_TRY(dev_alloc(S, (void**)&st.vlo, n * sizeof(float4)));
+    }
+    return LQ_OK;
+}
+
+/* T, and rec2 in its arrays' place (all but the stress, which the stress
+ * filter also uses).  T holds a state from the gather of a sort to its copy
+ * back, rec2 the boundary slots' records from the pack that ends the sort and
+ * the material slots' from stage 1 to stage 2 of a step: never at once. */
+int alloc_scratch_state(LqSim* S)
+{
+    const size_t n = (size_t)S->np;
+    LQ_TRY(dev_alloc(S, (void**)&S->T.pos, n * (3 * sizeof(float4) + sizeof(tensor2d))));
+    S->T.vel = S->T.pos + n;
+    S->T.idep = S->T.pos + 2 * n;
+    S->T.stn = reinterpret_cast<tensor2d*>(S->T.pos + 3 * n);
+    static_assert(3 * sizeof(float4) + sizeof(tensor2d) >= 13 * sizeof(float), "a record's words fit");
+    S->rec2 = reinterpret_cast<float*>(S->T.pos);       /* cudaMalloc: 256-byte aligned */
+    LQ_TRY(dev_alloc(S, (void**)&S->T.str, n * sizeof(tensor2d)));
+    if (S->flags & LQ_SIM_MIXED) {
+        LQ_TRY(dev_alloc(S, (void**)&S->T.xlo, n * sizeof(float4)));
+        LQ_TRY(dev_alloc(S, (void**)&S->T.vlo, n * sizeof(float4)));
     }
     return LQ_OK;
 }
@@ -732,7 +753,7 @@ int create(LqSim* S, const Parameters* par, const float* pos, const float* vel, 
     LQ_TRY(dev_alloc(S, (void**)&S->pd, sizeof(Parameters)));
     LQ_TRY(alloc_state(S, S->S));
     LQ_TRY(alloc_state(S, S->S2, S->S.idep));   /* the stage buffer shares the object words */
-    LQ_TRY(alloc_state(S, S->T));
+    LQ_TRY(alloc_scratch_state(S));
     const size_t n = (size_t)S->np;
     LQ_TRY(dev_alloc(S, (void**)&S->xbuild, n * sizeof(float4)));
     if (S->flags & LQ_SIM_DENSITY_FILTER) LQ_TRY(dev_alloc(S, (void**)&S->rho_f, n * sizeof(float)));
@@ -741,7 +762,6 @@ int create(LqSim* S, const Parameters* par, const float* pos, const float* vel, 
         LQ_TRY(dev_alloc(S, (void**)&S->dtime, sizeof(double)));
     }
     LQ_TRY(dev_alloc(S, (void**)&S->rec, n * 13 * sizeof(float)));   /* cudaMalloc: 256-byte aligned */
-    LQ_TRY(dev_alloc(S, (void**)&S->rec2, n * 13 * sizeof(float)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.accad, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.spin, n * sizeof(float4)));
     LQ_TRY(dev_alloc(S, (void**)&S->R.acestn, n * sizeof(tensor2d)));
