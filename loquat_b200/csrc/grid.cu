@@ -110,20 +110,28 @@ struct OrderOutputs {
     int* ident_out;
 };
 
-/* A warp takes kCells cells, one after the other: the lanes load a cell's slots
- * (the next cell's meanwhile), a vote tells whether they are in order, and
- * if not each lane finds its particle's place by counting the smaller ones.
- * One thread per cell, inserting, was a chain of about 17 dependent loads
- * and stores with most threads of a warp idle.  A search over 2.3 M
- * particles a few percent of which changed their cell takes 83 us instead of
- * 134, with the bounds and identities (23 us as kernels of their own) in
- * this pass.  A cell of more than 128 particles is ordered by one lane. */
+/* A warp orders kCells cells: lanes load the cells' slots (the next ones'
+ * meanwhile), a vote tells whether they are in order, and if not each lane
+ * finds its particle's place by counting the smaller ones.  The lanes that a
+ * cell gets follow the fullest of the warp's cells: with up to 16 particles
+ * each, 4, 8 or 16, so two to eight cells at a time; else all 32, and a cell
+ * of up to 128 in four loads.  A cell of more is ordered by its own lane,
+ * beside the warp's other such cells.  Bound by the chain of cells; a search
+ * over 2.3 M particles, 18 a cell, a few percent of which changed theirs, takes
+ * 84 us, of which bounds and identities (23 us as kernels of their own) are
+ * written here.
+ *
+ * Measured against one thread per cell that inserts (and against one cell at a
+ * time whatever its size), us a search over 2.0 M particles with 0.9, 1.9, 3.8,
+ * 16 and 128 a cell on average: 121, 82, 64, 54, 712; one thread per cell 125,
+ * 89, 74, 91, 1030; one cell at a time 182, 131, 88, 54, 2739. */
 template <int kCells>
 __global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, int np, const int* __restrict__ start, int* part_idx,
                                                        OrderOutputs out)
 {
+    __shared__ unsigned char full[kBlock / 32][32];     /* the warp's cells that hold particles */
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int first = (blockIdx.x * kBlock + threadIdx.x) / 32 * kCells;
     const int c = first + lane;
     int s = 0, n = 0;
@@ -140,63 +148,103 @@ __global__ void __launch_bounds__(kBlock) k_cell_order(int ncell, int np, const 
         if (out.ident_out) out.ident_out[d] = !lq_in_range(v, np) ? -1 : out.ident_in ? __ldg(out.ident_in + v) : v;
     };
     unsigned todo = __ballot_sync(FULL, n > 0);
-    int k = __ffs((int)todo) - 1;
-    int cs = __shfl_sync(FULL, s, k & 31), cn = __shfl_sync(FULL, n, k & 31);
-    int v = todo && lane < cn ? part_idx[cs + lane] : INT_MAX;
-    while (todo) {
-        todo &= todo - 1;
-        const int k2 = __ffs((int)todo) - 1;
-        const int s2 = __shfl_sync(FULL, s, k2 & 31), n2 = __shfl_sync(FULL, n, k2 & 31);
-        const int v2 = todo && lane < n2 ? part_idx[s2 + lane] : INT_MAX;
-        const int cell = first + k;
-        if (cn <= 32) {
-            const int after = __shfl_down_sync(FULL, v, 1);
-            int r = lane;
-            if (__any_sync(FULL, lane + 1 < cn && v > after)) {
+    unsigned big = 0;
+    if (!__any_sync(FULL, n > 16)) {
+        if (n > 0) full[w][__popc(todo & ((1u << lane) - 1u))] = (unsigned char)lane;
+        __syncwarp();
+        const int cells = __popc(todo);
+        const int most = __reduce_max_sync(FULL, n);
+        const int W = most <= 4 ? 4 : most <= 8 ? 8 : 16;
+        const int sub = lane & (W - 1), per = 32 / W;
+        int q = lane / W, at = 0, cs = 0, cn = 0, v = INT_MAX;
+        auto take = [&]() {
+            at = q < cells ? full[w][q] : 0;
+            cs = __shfl_sync(FULL, s, at);
+            cn = __shfl_sync(FULL, n, at);
+            if (q >= cells) cn = 0;
+            v = sub < cn ? part_idx[cs + sub] : INT_MAX;
+            q += per;
+        };
+        take();
+        for (int base = 0; base < cells; base += per) {
+            const int at0 = at, cs0 = cs, cn0 = cn, v0 = v;
+            take();
+            const int after = __shfl_down_sync(FULL, v0, 1, W);
+            int r = sub;
+            if (__any_sync(FULL, sub + 1 < cn0 && v0 > after)) {
                 r = 0;
-                for (int q = 0; q < cn; ++q) r += __shfl_sync(FULL, v, q) < v;
-                if (lane < cn) part_idx[cs + r] = v;
+                for (int o = 0; o < W; ++o) r += __shfl_sync(FULL, v0, o, W) < v0;
+                if (sub < cn0) part_idx[cs0 + r] = v0;
             }
-            if (lane < cn) place(cs + r, v, cell);
-        } else if (cn <= 128) {
-            int w[4], r[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                w[u] = 32 * u + lane < cn ? part_idx[cs + 32 * u + lane] : INT_MAX;
-                r[u] = 0;
-            }
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                for (int q = 0; q < 32; ++q) {
-                    const int o = __shfl_sync(FULL, w[b], q);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) r[u] += o < w[u];
-                }
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (32 * u + lane < cn) {
-                    part_idx[cs + r[u]] = w[u];
-                    place(cs + r[u], w[u], cell);
-                }
-        } else {
-            if (lane == 0)
-                for (int a = cs + 1; a < cs + cn; ++a) {
-                    const int x = part_idx[a];
-                    int b = a - 1;
-                    while (b >= cs && part_idx[b] > x) {
-                        part_idx[b + 1] = part_idx[b];
-                        --b;
-                    }
-                    part_idx[b + 1] = x;
-                }
-            __syncwarp();
-            for (int d = cs + lane; d < cs + cn; d += 32) place(d, part_idx[d], cell);
+            if (sub < cn0) place(cs0 + r, v0, first + at0);
         }
-        k = k2;
-        cs = s2;
-        cn = n2;
-        v = v2;
+    } else {
+        big = __ballot_sync(FULL, n > 128);
+        todo &= ~big;
+        int k = __ffs((int)todo) - 1;
+        int cs = __shfl_sync(FULL, s, k & 31), cn = __shfl_sync(FULL, n, k & 31);
+        int v = todo && lane < cn ? part_idx[cs + lane] : INT_MAX;
+        while (todo) {
+            todo &= todo - 1;
+            const int k2 = __ffs((int)todo) - 1;
+            const int s2 = __shfl_sync(FULL, s, k2 & 31), n2 = __shfl_sync(FULL, n, k2 & 31);
+            const int v2 = todo && lane < n2 ? part_idx[s2 + lane] : INT_MAX;
+            const int cell = first + k;
+            if (cn <= 32) {
+                const int after = __shfl_down_sync(FULL, v, 1);
+                int r = lane;
+                if (__any_sync(FULL, lane + 1 < cn && v > after)) {
+                    r = 0;
+                    for (int o = 0; o < cn; ++o) r += __shfl_sync(FULL, v, o) < v;
+                    if (lane < cn) part_idx[cs + r] = v;
+                }
+                if (lane < cn) place(cs + r, v, cell);
+            } else {
+                int u4[4], r[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    u4[u] = 32 * u + lane < cn ? part_idx[cs + 32 * u + lane] : INT_MAX;
+                    r[u] = 0;
+                }
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    for (int o = 0; o < 32; ++o) {
+                        const int x = __shfl_sync(FULL, u4[b], o);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) r[u] += x < u4[u];
+                    }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (32 * u + lane < cn) {
+                        part_idx[cs + r[u]] = u4[u];
+                        place(cs + r[u], u4[u], cell);
+                    }
+            }
+            k = k2;
+            cs = s2;
+            cn = n2;
+            v = v2;
+        }
+    }
+    if (!big) return;
+    if (n > 128) {
+        bool sorted = true;     /* most arrive in order: a read-only pass leaves them alone */
+        for (int a = s + 1; a < s + n && sorted; ++a) sorted = part_idx[a - 1] < part_idx[a];
+        for (int a = s + 1; a < s + n && !sorted; ++a) {
+            const int x = part_idx[a];
+            int b = a - 1;
+            while (b >= s && part_idx[b] > x) {
+                part_idx[b + 1] = part_idx[b];
+                --b;
+            }
+            part_idx[b + 1] = x;
+        }
+    }
+    __syncwarp();
+    for (unsigned m = big; m; m &= m - 1) {
+        const int k = __ffs((int)m) - 1, cs = __shfl_sync(FULL, s, k), cn = __shfl_sync(FULL, n, k);
+        for (int d = cs + lane; d < cs + cn; d += 32) place(d, part_idx[d], first + k);
     }
 }
 
