@@ -1032,21 +1032,30 @@ __global__ void __launch_bounds__(128) k_interaction_group(const Parameters* __r
 /* The sums of the reference's two kernels that walk the material layer
  * (src/adami_boundary.cu:27-123, src/field_smoothing.cu:65-121): sigma_j
  * V_j W in S, x_ij V_j W and V_j W in acc, over the 27 cells around a
- * target.  Eight
- * lanes share a target: they test its candidates eight (two times eight) at
- * a time, queue those within 2h in shared memory and then form the terms of
- * eight queued ones at once, so the square root, the quotient and the loads
- * of a term are done by full groups; one thread per target ran them for the
- * one candidate in six that passed, with the other lanes waiting, as a
- * chain of dependent loads (8 warps per SM in the wall's case).  Bound by
- * issue slots (77 %), so a term's distance is a plain square root of the
- * squared sum (norm3df, which guards against overflow of the squares, cost
- * 18 us of 400) and its two factors are multiplied once.  The wall of 116 k
- * particles takes 22.8 us instead of 84, the filter over 402 k soil
- * particles 377 instead of 674; groups that voted and looped each by
- * themselves ran one after another (754). */
+ * target.  Eight lanes share a target: they test its candidates eight (two
+ * times eight) at a time, queue those within 2h in shared memory and then
+ * form the terms of eight queued ones at once, so the square root, the
+ * quotient and the loads of a term are done by full groups; one thread per
+ * target ran them for the one candidate in six that passed, with the other
+ * lanes waiting, as a chain of dependent loads (8 warps per SM in the wall's
+ * case).  Bound by issue slots (78 %), so a term's distance is a plain square
+ * root of the squared sum (norm3df, which guards against overflow of the
+ * squares, cost 18 us of 400) and its two factors are multiplied once.  The
+ * wall of 116 k particles takes 20.6 us instead of 84, the filter over 402 k
+ * soil particles 376 instead of 674; groups that voted and looped each by
+ * themselves ran one after another (754).
+ *
+ * Where every target of a warp has at most kCellFew candidates, testing them
+ * column by column leaves most lanes idle: they are queued untested, and a
+ * warp without any ends there.  A sheet of 1 M particles in one layer with 1.4,
+ * 2.6 and 4 a cell: filter 147, 167 and 202 us so, 225, 240 and 242 column by
+ * column; up to 32 or 64 candidates instead of 40 it is slower for 36, or for
+ * 61.  One thread per target is still faster there (119, 142 and 190 us),
+ * where latency is hidden by many targets, but by far the slower one with
+ * fewer targets or more candidates. */
 constexpr int kCellLanes = 8;
 constexpr int kCellQueue = 64;
+constexpr int kCellFew = 40;
 
 struct CellSums {
     tensor2d S;
@@ -1129,47 +1138,66 @@ __device__ __forceinline__ CellSums sum_material_cells(const Parameters* __restr
     /* lane g finds the slots of column g of the 3 x 3 (lane 0 also those of
      * column 8): one range while the column's cells follow one another in
      * the slots, as they do in a grid sorted by the cell key */
-    for (int first = 0; first < 9; first += kCellLanes) {
-        const int col = first + g;
+    int s0[2] = {0, 0}, e0[2] = {0, 0};
+    bool apart[2] = {false, false};
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int col = t * kCellLanes + g;
         const int X = cx + col % 3 - 1, Y = cy + col / 3 - 1;
-        int s = 0, e = 0;
-        bool apart = false;
-        if (col < 9 && X >= 0 && X < nx && Y >= 0 && Y < ny) {
-            const int cell = L + (X * ny + Y) * nz + zlo;
-            int b[3], f[3];
+        if (col >= 9 || X < 0 || X >= nx || Y < 0 || Y >= ny) continue;
+        const int cell = L + (X * ny + Y) * nz + zlo;
+        int b[3], f[3];
 #pragma unroll
-            for (int z = 0; z < 3; ++z) {
-                const bool in = zlo + z <= zhi;
-                b[z] = in ? __ldg(cells.beg + cell + z) : -1;
-                f[z] = in ? __ldg(cells.end + cell + z) : -1;
-            }
-#pragma unroll
-            for (int z = 0; z < 3; ++z) {
-                if (b[z] == -1 || f[z] <= b[z]) continue;   /* empty, by either mark */
-                if (e == 0) {
-                    s = b[z];
-                } else if (b[z] != e) {
-                    apart = true;
-                }
-                e = f[z];
-            }
+        for (int z = 0; z < 3; ++z) {
+            const bool in = zlo + z <= zhi;
+            b[z] = in ? __ldg(cells.beg + cell + z) : -1;
+            f[z] = in ? __ldg(cells.end + cell + z) : -1;
         }
-        const bool any_apart = __any_sync(FULL, apart);
-        for (int c = 0; c < kCellLanes && first + c < 9; ++c) {
-            const int cs = __shfl_sync(FULL, s, c, kCellLanes), ce = __shfl_sync(FULL, e, c, kCellLanes);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+            if (b[z] == -1 || f[z] <= b[z]) continue;   /* empty, by either mark */
+            if (e0[t] == 0) {
+                s0[t] = b[z];
+            } else if (b[z] != e0[t]) {
+                apart[t] = true;
+            }
+            e0[t] = f[z];
+        }
+    }
+    const bool any_apart = __any_sync(FULL, apart[0] || apart[1]);
+    const int len = e0[0] - s0[0];
+    int upto = len;     /* of this lane's and the lanes' before it */
+#pragma unroll
+    for (int o = 1; o < kCellLanes; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, upto, o, kCellLanes);
+        if (g >= o) upto += v;
+    }
+    const int eight = __shfl_sync(FULL, upto, kCellLanes - 1, kCellLanes);
+    const int last = __shfl_sync(FULL, s0[1], 0, kCellLanes), last_len = __shfl_sync(FULL, e0[1], 0, kCellLanes) - last;
+    if (!any_apart && __all_sync(FULL, eight + last_len <= kCellFew)) {
+        /* few candidates: all of them queued untested */
+        if (!__any_sync(FULL, eight + last_len > 0)) return r;
+        for (int k = 0; __any_sync(FULL, k < len); ++k)
+            if (k < len) queue[upto - len + k] = s0[0] + k;
+        for (int k = g; k < last_len; k += kCellLanes) queue[eight + k] = last + k;
+        n = eight + last_len;
+    } else {
+        for (int c = 0; c < 9; ++c) {
+            const int t = c / kCellLanes, l = c % kCellLanes;
+            const int cs = __shfl_sync(FULL, t ? s0[1] : s0[0], l, kCellLanes);
+            const int ce = __shfl_sync(FULL, t ? e0[1] : e0[0], l, kCellLanes);
             if (!any_apart) {
                 if (__any_sync(FULL, cs < ce)) test(cs, ce);
                 continue;
             }
             /* some column's cells are apart: every column cell by cell */
-            const bool cell_by_cell = __shfl_sync(FULL, (int)apart, c, kCellLanes);
-            const int k = first + c;
+            const bool cell_by_cell = __shfl_sync(FULL, (int)(t ? apart[1] : apart[0]), l, kCellLanes);
             for (int dz = 0; dz < 3; ++dz) {
                 int b = dz == 0 ? cs : 0, f = dz == 0 ? ce : 0;
                 if (cell_by_cell) {
                     const int z = zlo + dz;
                     b = f = 0;
-                    if (z > zhi || !cell_range(cells, L + ((cx + k % 3 - 1) * ny + cy + k / 3 - 1) * nz + z, b, f))
+                    if (z > zhi || !cell_range(cells, L + ((cx + c % 3 - 1) * ny + cy + c / 3 - 1) * nz + z, b, f))
                         b = f = 0;
                 }
                 test(b, f);
