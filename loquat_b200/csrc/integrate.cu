@@ -111,7 +111,10 @@ __global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_trial(const Par
  * evaluates a rate in every turn.  The particles whose step was cut most
  * come first, since the longest chain of evaluations ends the launch.
  * Bound by FP64 latency, and in small cases by the longest chain: 64
- * trials of two evaluations take 150 us. */
+ * trials of two evaluations take 150 us where a warp has its part of the SM to
+ * itself.  A short queue is therefore left to as many blocks as it fills, which
+ * lie on different SMs; whichever warps came first took it otherwise, on a few
+ * SMs (5 k particles with up to 64 sub-steps each: 840 us a step, so 564). */
 __global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_finish(const Parameters* __restrict__ P, double part,
                                                                         const float4* idep,
                                                                         const tensor2d* src_str, State out,
@@ -122,6 +125,7 @@ __global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_finish(const Pa
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int nhard = q.counts[0], n = nhard + q.counts[1];
+    if ((long long)blockIdx.x * kBlock >= n) return;
     const double dt = part * (double)__ldg(&P->dt);
     int i = -1;
     bool drained = false;
