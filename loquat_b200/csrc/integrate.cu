@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_trial(const Par
     if (lane == leader) at = atomicAdd(q.counts + (hard ? 0 : 1), __popc(peers));
     at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
     if (!hard) at = q.cap - 1 - at;
+    if (!lq_in_range(at, q.cap)) return;
     q.item[at] = i;
     q.h[at] = g.h;
 }
@@ -142,12 +143,16 @@ __global__ void __launch_bounds__(kBlock, LQ_VW_MIN_BLOCKS) k_vw_finish(const Pa
             if (idle >> lane & 1u) {
                 if (at < n) {
                     if (at >= nhard) at = q.cap - 1 - (at - nhard);
-                    i = q.item[at];
-                    const float4 id = idep[i];
-                    c = vw_row(vw, id.x);
-                    w = __ldg(rt.spin + i);
-                    de = load_t2(rt.acestn, i);
-                    g.start(widen6(load_t2_rw(src_str, i)), id.z, de, q.h[at], 1);
+                    if (lq_in_range(at, q.cap)) i = q.item[at];
+                    if (lq_in_range(i, __ldg(&P->np))) {
+                        const float4 id = idep[i];
+                        c = vw_row(vw, id.x);
+                        w = __ldg(rt.spin + i);
+                        de = load_t2(rt.acestn, i);
+                        g.start(widen6(load_t2_rw(src_str, i)), id.z, de, q.h[at], 1);
+                    } else {
+                        i = -1;
+                    }
                 } else {
                     drained = true;
                 }
@@ -219,6 +224,18 @@ __global__ void __launch_bounds__(kBlock, LQ_INT_MIN_BLOCKS) k_correct(const Par
 }
 
 }  // namespace
+
+/* This translation unit's count of bounds violations (always 0 without
+ * LQ_CHECKED). */
+int bounds_count_integrate(unsigned long long* v)
+{
+#ifdef LQ_CHECKED
+    LQ_TRY_CUDA(cudaMemcpyFromSymbol(v, lq_bounds_count, sizeof(*v)), "bounds counter");
+#else
+    *v = 0;
+#endif
+    return LQ_OK;
+}
 
 size_t vw_row_bytes() { return sizeof(VWConst); }
 

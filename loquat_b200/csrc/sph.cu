@@ -486,7 +486,8 @@ __global__ void __launch_bounds__(kBlock) k_neighbor_list(const Parameters* __re
             float4 x[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                x[c] = j[c] >= 0 ? __ldg(pos + j[c]) : make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f);
+                x[c] = j[c] >= 0 && lq_in_range(j[c], np_all) ? __ldg(pos + j[c])
+                                                              : make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f);
                 slot[w][32 * c + lane] = j[c];
             }
             float2 mx[2], my[2], mz[2];
@@ -702,6 +703,7 @@ __global__ void __launch_bounds__(kArrangeBlock) k_list_arrange(int ntarget, con
             for (int o = 0; o < 8; ++o) row[o] = hd[(w + o) & 7][x];
 #pragma unroll
             for (int o = 0; o < 8; ++o) {
+                if (!lq_in_range(row[o], m)) continue;
                 const unsigned char next = nxt[row[o]][x];
                 p[(size_t)(k + o) * stride] = ent[row[o]][x];
                 hd[(w + o) & 7][x] = next;
@@ -712,6 +714,7 @@ __global__ void __launch_bounds__(kArrangeBlock) k_list_arrange(int ntarget, con
             const int w = (t + base + k) & 7;
             const int r = (w + __ffs((int)((have | have << 8) >> w)) - 1) & 7;
             const int row = hd[r][x];
+            if (!lq_in_range(row, m)) break;
             const unsigned char next = nxt[row][x];
             p[(size_t)k * stride] = ent[row][x];
             hd[r][x] = next;
@@ -830,6 +833,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
     int row = t, self = i;
     if (kStage == 0 && rows) {
         row = __ldg(rows + t);
+        if (!lq_in_range(row + 1, np - npb + 1)) row = -1;
         self = npb + row;
     }
     const int n = row >= 0 ? __ldg(count + row) : LQ_NBR_CAP + 1;
@@ -2283,10 +2287,11 @@ extern "C" int lq_debug_bounds_violations(long long* count)
     if (!count) return lqb::set_error(LQ_ERR_ARG, "lq_debug_bounds_violations: null argument");
 #ifdef LQ_CHECKED
     LQ_TRY_CUDA(cudaDeviceSynchronize(), "bounds counter");
-    unsigned long long a = 0, b = 0;
+    unsigned long long a = 0, b = 0, c = 0;
     LQ_TRY(lqb::bounds_count_sph(&a));
     LQ_TRY(lqb::bounds_count_grid(&b));
-    *count = (long long)(a + b);
+    LQ_TRY(lqb::bounds_count_integrate(&c));
+    *count = (long long)(a + b + c);
 #else
     *count = -1;
 #endif
