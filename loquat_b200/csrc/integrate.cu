@@ -6,9 +6,11 @@
  * The reference issues five device-to-device snapshot copies and then the
  * predictor kernel; here the snapshot is written by the same kernel that
  * reads the state, so the state is read once.  The native driver skips the
- * snapshot entirely: the predictor writes into a second buffer and the
- * corrector reads the untouched first buffer through the new sort
- * permutation.
+ * snapshot entirely: the predictor step writes into a second buffer and the
+ * corrector step restarts from the untouched first one, in place.  Its
+ * thread-per-target pair kernels take both steps themselves (sph.cu); the
+ * kernels here serve the drop-in calls, the warp-cooperative pair shapes and,
+ * for every shape, model 3's stresses.
  */
 #include <cstdio>
 #include <cstdlib>
@@ -29,12 +31,12 @@ constexpr int kBlock = 128;
 #ifndef LQ_VW_MIN_BLOCKS
 #define LQ_VW_MIN_BLOCKS 4
 #endif
-/* resident blocks per SM asked of the other instantiations: 6 caps them at
- * 80 registers (the mixed form's FP64 return map spills ~130 B), 24 warps
- * per SM instead of 16 for the uncapped 117-120; on the 256-scenario
- * ensemble the mixed integrators took 2.19 ms per step against 2.25 (5),
- * 2.22 (7), 2.36 (8) and 2.49 uncapped; the plain ones (78 registers) are
- * unaffected */
+/* resident blocks per SM asked of k_predict and k_correct: 6 caps them at 80
+ * registers (the mixed form's FP64 return map spills), 24 warps per SM instead
+ * of 16 uncapped (117 to 120); when the native driver still integrated by
+ * them in every shape, the 256-scenario ensemble's mixed integrations took
+ * 2.19 ms a step against 2.25 (5), 2.22 (7), 2.36 (8) and 2.49 uncapped; the
+ * plain ones (78 registers) are unaffected */
 #ifndef LQ_INT_MIN_BLOCKS
 #define LQ_INT_MIN_BLOCKS 6
 #endif
@@ -206,21 +208,18 @@ __global__ void __launch_bounds__(kBlock, LQ_INT_MIN_BLOCKS) k_predict(const Par
     predict_slot<kMixed>(P, i, in, out, load_rates(rt, i), mt, nb, stage, x0, v0, id, s0, e0);
 }
 
-/* Corrector of the material slots from the snapshot `ini` (at ini_idx[i],
- * or i) and the current state `cur` into `out` (which may be either). */
+/* Corrector of the material slots from the snapshot `ini` and the current
+ * state `cur` into `out` (which may be either); boundary slots are Adami's. */
 template <bool kMixed>
 __global__ void __launch_bounds__(kBlock, LQ_INT_MIN_BLOCKS) k_correct(const Parameters* __restrict__ P, int np,
-                                                                       int npb, State cur, State ini,
-                                                                       const int* __restrict__ ini_idx, State out,
+                                                                       int npb, State cur, State ini, State out,
                                                                        Rates rt, int* __restrict__ health,
-                                                                       VerletCheck verlet, int first,
-                                                                       MaterialTable mt, NbrArrays nb)
+                                                                       VerletCheck verlet, MaterialTable mt,
+                                                                       NbrArrays nb)
 {
-    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = npb + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    if (i < npb) return;    /* boundary slots: Adami writes both buffers */
-    const int k = ini_idx ? __ldg(ini_idx + i) : i;
-    correct_slot<kMixed>(P, i, k, cur.pos[i].w, cur.idep[i], ini, out, load_rates(rt, i), mt, nb, health, verlet);
+    correct_slot<kMixed>(P, i, cur.pos[i].w, cur.idep[i], ini, out, load_rates(rt, i), mt, nb, health, verlet);
 }
 
 }  // namespace
@@ -318,15 +317,15 @@ int launch_predict(const Parameters* ph, const Parameters* pd, const State& in, 
     return launch_predict_substeps(ph, pd, in, out, r, s, vw, rec, q);
 }
 
-int launch_correct(const Parameters* ph, const Parameters* pd, const State& cur, const State& ini,
-                   const int* ini_idx, const Rates& r, int* health, cudaStream_t s)
+int launch_correct(const Parameters* ph, const Parameters* pd, const State& cur, const State& ini, const Rates& r,
+                   cudaStream_t s)
 {
     if (ph->npm <= 0) return LQ_OK;
     if (ph->constitutive_model == 3)
         return set_error(LQ_ERR_ARG, "corrector: constitutive model 3 needs a von Wolffersdorff table");
     k_correct<false><<<blocks_for(ph->npm, kBlock), kBlock, 0, s>>>(
-        pd, ph->np, ph->npb, cur, ini, ini_idx, cur, r, health, VerletCheck{nullptr, nullptr, 0.0f, 0.0f, nullptr, 0.0f},
-        ph->npb, MaterialTable(), NbrArrays{nullptr, nullptr, nullptr});
+        pd, ph->np, ph->npb, cur, ini, cur, r, nullptr, VerletCheck{nullptr, nullptr, 0.0f, 0.0f, nullptr, 0.0f},
+        MaterialTable(), NbrArrays{nullptr, nullptr, nullptr});
     LQ_TRY_CUDA(cudaGetLastError(), "k_correct");
     return LQ_OK;
 }
@@ -340,14 +339,12 @@ int launch_correct_into(const Parameters* ph, const Parameters* pd, const State&
     if (lists.xwide && !(lists.wide > lists.skin))
         return set_error(LQ_ERR_ARG, "corrector: the wide cut-off must exceed the skin");
     const VerletCheck vc = verlet_of(ph, lists);
-    /* material slots only: boundary slots are written by Adami into both
-     * buffers */
-    const int nb = blocks_for(ph->npm, kBlock), f = ph->npb;
+    const int nb = blocks_for(ph->npm, kBlock);
     const NbrArrays pk = rec ? nbr_arrays(rec, ph->np) : NbrArrays{nullptr, nullptr, nullptr};
     if (ini.xlo)
-        k_correct<true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, ini, r, health, vc, f, mt, pk);
+        k_correct<true><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, ini, r, health, vc, mt, pk);
     else
-        k_correct<false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, nullptr, ini, r, health, vc, f, mt, pk);
+        k_correct<false><<<nb, kBlock, 0, s>>>(pd, ph->np, ph->npb, cur, ini, ini, r, health, vc, mt, pk);
     LQ_TRY_CUDA(cudaGetLastError(), "k_correct");
     return launch_correct_substeps(ph, pd, ini, r, health, s, vw, rec, q);
 }
@@ -390,7 +387,7 @@ extern "C" int lq_corrector(const void* par_host, const void* par_device, float*
     lqb::State in{(float4*)pospres_ini, (float4*)velrhop_ini, (float4*)idep_ini, (tensor2d*)str_ini,
                   (tensor2d*)stn_ini};
     lqb::Rates r{(float4*)accad, (float4*)spin, (tensor2d*)acestn};
-    return lqb::launch_correct(ph, static_cast<const Parameters*>(par_device), st, in, nullptr, r, nullptr,
+    return lqb::launch_correct(ph, static_cast<const Parameters*>(par_device), st, in, r,
                                static_cast<cudaStream_t>(stream));
 }
 

@@ -171,7 +171,7 @@ __device__ __forceinline__ void predict_slot(const Parameters* __restrict__ P, i
     pack_slot<kMixed>(nb, i, x, v, s);
 }
 
-/* Full step of material slot i from the snapshot `ini` at slot k
+/* Full step of material slot i from the snapshot `ini`
  * (reference src/predictor_corrector.cu:256-307): v = v0 + dt a;
  * x = x0 + dt/2 (v + v0); eps = eps0 + dt deps; the model restarts from the
  * snapshot's stress and plastic strain; the pressure passed in, p_now, is
@@ -179,24 +179,24 @@ __device__ __forceinline__ void predict_slot(const Parameters* __restrict__ P, i
  * results in health, and with `verlet` checks the lists.  Model 3's stress
  * and void ratio are k_vw_trial's, as above. */
 template <bool kMixed>
-__device__ __forceinline__ void correct_slot(const Parameters* __restrict__ P, int i, int k, float p_now,
+__device__ __forceinline__ void correct_slot(const Parameters* __restrict__ P, int i, float p_now,
                                              const float4& id, const State& ini, const State& out,
                                              const SlotRates& r, const MaterialTable& mt, const NbrArrays& nb,
                                              int* __restrict__ health, const VerletCheck& verlet)
 {
     const float dt = __ldg(&P->dt);
-    const float4 x0 = ini.pos[k];
-    const float4 v0 = ini.vel[k];
-    const float ep0 = ini.idep[k].y;
-    const tensor2d s0 = load_t2_rw(ini.str, k);
-    const tensor2d e0 = load_t2_rw(ini.stn, k);
+    const float4 x0 = ini.pos[i];
+    const float4 v0 = ini.vel[i];
+    const float ep0 = ini.idep[i].y;
+    const tensor2d s0 = load_t2_rw(ini.str, i);
+    const tensor2d e0 = load_t2_rw(ini.stn, i);
     const Material M = particle_material(load_material(P), mt, id.x);
     float4 v, x;
     tensor2d s = s0, e;
     float ep;
     if (kMixed) {
         const double ddt = dt;
-        const double4 v0d = join4(v0, ini.vlo[k]), x0d = join4(x0, ini.xlo[k]);
+        const double4 v0d = join4(v0, ini.vlo[i]), x0d = join4(x0, ini.xlo[i]);
         double4 vd, xd;
         vd.x = v0d.x + ddt * r.a.x; vd.y = v0d.y + ddt * r.a.y; vd.z = v0d.z + ddt * r.a.z; vd.w = v0d.w + ddt * r.a.w;
         xd.x = 0.5 * (vd.x + v0d.x) * ddt + x0d.x;

@@ -270,10 +270,9 @@ int launch_predict(const Parameters* par_host, const Parameters* par_dev, const 
                    const State* snap, const Rates& r, cudaStream_t s, const MaterialTable& mt = MaterialTable(),
                    const MaterialTable& vw = MaterialTable(), float* rec = nullptr, bool stage = false,
                    const SubstepQueue& q = SubstepQueue());
-/* Corrector in place on `cur`; ini values read at ini_idx[i] (identity when
- * ini_idx is null).  Non-finite results are counted in health. */
+/* Corrector in place on `cur` from the snapshot `ini`. */
 int launch_correct(const Parameters* par_host, const Parameters* par_dev, const State& cur, const State& ini,
-                   const int* ini_idx, const Rates& r, int* health, cudaStream_t s);
+                   const Rates& r, cudaStream_t s);
 
 /* Corrector from the snapshot `ini` and the current stage buffer `cur` into
  * `ini`, material slots only; material particles raise bit 1 of *flag when

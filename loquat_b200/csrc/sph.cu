@@ -52,11 +52,11 @@ inline int blocks_for(long long n, int b) { return (int)((n + b - 1) / b); }
  * mu = h v_ij.x_ij / (r^2 + eta) for approaching pairs; R is the diagonal
  * artificial stress -eps sig_aa / rho^2 of tensile components, f = W/W(dr).
  *
- * Neighbours are visited through lists: k_neighbor_list walks the union
- * of a warp's lanes' 27-cell stencils in lockstep (one broadcast load per
- * candidate, one distance test per lane) and writes each lane's hits to a
- * global list in coalesced rows; the pair kernels then evaluate each
- * particle's pairs from its list with every lane busy.  The native driver
+ * Neighbours are visited through lists: k_neighbor_list holds the candidates
+ * of a warp's targets in its lanes, tests them against one target after the
+ * other and writes each target's hits to its column of a global list; the
+ * pair kernels then evaluate each particle's pairs from its list with every
+ * lane busy.  The native driver
  * keeps the lists across steps (Verlet lists with a skin); the drop-in
  * ParticleInteraction builds them at each call in the caller's grid.  A
  * particle whose list overflowed walks its stencil directly (walk_stencil),
@@ -795,7 +795,7 @@ __device__ __forceinline__ void integrate_target(const Parameters* __restrict__ 
         predict_slot<kKahan>(P, i, tail.in, tail.out, r, tail.mt, tail.nbw, true, tail.in.pos[i], tail.in.vel[i],
                              tail.in.idep[i], load_t2_rw(tail.in.str, i), make_tensor2d(0.0f));
     else
-        correct_slot<kKahan>(P, i, i, __ldg(&st.pos[i].w), tail.in.idep[i], tail.in, tail.in, r, tail.mt, tail.nbw,
+        correct_slot<kKahan>(P, i, __ldg(&st.pos[i].w), tail.in.idep[i], tail.in, tail.in, r, tail.mt, tail.nbw,
                              tail.health, tail.verlet);
 }
 
@@ -811,7 +811,10 @@ __device__ __forceinline__ void integrate_target(const Parameters* __restrict__ 
  * kernels of their own (131 us each after pair launches of 605), the
  * 5 k column 69 and 75.  The
  * step writes the records that the next stage gathers, so the two stages'
- * records are separate arrays: this one's are still being read. */
+ * records are separate arrays: this one's are still being read.  At 80
+ * registers the mixed form spills 76 bytes (stage 1) and 156 (stage 2), all
+ * in the FP64 integration after the sums; at 96 24 and 88, at 72 160 and 244.
+ * The plain form spills none. */
 template <bool kKahan, int kThreads, int kMinBlocks, int kStage>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
     const Parameters* __restrict__ P, int np, int npb, State st, Rates rt, Cells cells, const int* __restrict__ list,
@@ -856,7 +859,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_interaction_rec(
  * sums of the thread-per-target form bit for bit.  A thread's list of about
  * 80 entries is a chain of 20 groups of dependent gathers and about 8000
  * instructions; below some 30 k targets there are too few warps to hide it
- * and the launch takes 19 us whatever its size.  Here each lane forms the
+ * and the launch takes 23 us however few there are.  Here each lane forms the
  * factors of one entry in 16 (the bulk of the work, in any order) and puts
  * them into shared memory; then the lanes each own one of the target's 13
  * sums and add the 16 terms in the list's order, in the groups of four of
@@ -1303,7 +1306,8 @@ __device__ __forceinline__ void store_wall_stress(const Parameters* __restrict__
  * more than kAdamiLanes, or four to twice that, else one: 9.3 us at the 5 k
  * column (11.3 with 4, 16 with 1), 18.2 with 4 at the 1.97 M cylinder's 70 k
  * targets (21.0 with 8, 23.7 with 1), 44 with 1 at the 2.85 M slope (64 with
- * 2, 88 with 8).  The launch has a lane for every boundary particle, and
+ * 2, 88 with 8).  Between 65 k and 131 k targets either of one and four lanes
+ * is up to 5 us the better one, with the lists' lengths.  The launch has a lane for every boundary particle, and
  * eight up to kAdamiLanes; blocks beyond the targets end at once (a grid of
  * 12 blocks per SM that strides: 52 us at the slope).
  *
@@ -1801,8 +1805,9 @@ int launch_shepard_list(const Parameters* ph, const Parameters* pd, const State&
 
 namespace {
 
-/* Shape 0 gives each target a team of lanes up to this many: between the
- * 5 k and 12 k at which the two forms were measured (k_interaction_team). */
+/* Shape 0 gives each target a team of lanes up to this many (us a step with
+ * teams and without, plain; mixed): 8000 targets 43.7 and 57.4; 53.2 and 57.5,
+ * 9600 53.5 and 57.2; 57.5 and 57.5, 12000 55.6 and 58.0; 67.7 and 59.5. */
 #ifndef LQ_TEAM_TARGETS
 #define LQ_TEAM_TARGETS 8192
 #endif
