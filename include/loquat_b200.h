@@ -59,18 +59,20 @@ int lq_grid_resize(void* grid, int np, int ncell);
 int lq_grid_destroy(void* grid);
 /* Hash, stable sort and cell bounds (LoquatGrid::NeighborSearch,
  * reference src/loquat_grid.h:60).  pospres/idep: device float4[np].  The
- * stable order within a cell is restored by one thread per cell, in one
- * read-only pass when the cell arrives in order (as it does when particles
- * move little between searches) and by insertion otherwise: particles
- * outside the lattice share one cell, so keep their number small. */
+ * stable order within a cell is restored by a group of threads, or for
+ * more than 128 particles by one thread: in one read-only pass when the cell
+ * arrives in order (as it does when particles move little between searches)
+ * and by insertion otherwise.  Particles outside the lattice share one cell,
+ * so keep their number small. */
 int lq_grid_neighbor_search(void* grid, const void* par_host, const void* par_device,
                             const float* pospres, const float* idep, void* stream);
 /* Device pointers owned by the grid.  cell_start has ncell + 1 entries:
  * the particles of cell c are the sorted slots [cell_start[c], cell_start[c+1]). */
 int lq_grid_arrays(void* grid, const int** part_cel, const int** part_idx,
                    const int** cell_beg, const int** cell_end, const int** cell_start);
-/* data[i] <- data[part_idx[i]] through cache (LoquatGrid::SortArrayFloat4 /
- * SortArrayTensor2d, reference src/loquat_grid.h:62-64). */
+/* data[i] <- data[part_idx[i]] through cache, which holds the sorted array
+ * too afterwards (LoquatGrid::SortArrayFloat4 / SortArrayTensor2d, reference
+ * src/loquat_grid.h:62-64). */
 int lq_grid_sort_float4(void* grid, int np, float* data, float* cache, void* stream);
 int lq_grid_sort_tensor2d(void* grid, int np, float* data, float* cache, void* stream);
 
@@ -98,8 +100,8 @@ int lq_grid_neighbor_search_noalloc(const void* par_host, const void* par_device
 
 /* ---- per-stage operators ------------------------------------------------ */
 /* Sizes the working arrays of lq_particle_interaction on the current device
- * (cell starts, target order, neighbour lists, packed neighbour data) for
- * the particle and cell counts of par_host.  No counterpart in the
+ * (neighbour lists, packed neighbour data, what carries them from call to
+ * call) for the particle counts of par_host.  No counterpart in the
  * reference, whose ParticleInteraction is closed; it plays the part of the
  * reference's set-up allocation (src/loquat.cu:142-165) for this
  * operator: the drop-in LoquatGrid::GridConfig calls it, and a C caller
@@ -119,7 +121,9 @@ int lq_interaction_reserve(const void* par_host);
  * the grid's searches and the interaction must run on one stream. */
 int lq_interaction_stats(long long* rebuilds, long long* reuses);
 
-/* reference src/particle_interaction.h:27-40 */
+/* reference src/particle_interaction.h:27-40.  The particles lie cell by
+ * cell in the order of the cell key, as a search leaves them; an empty cell
+ * has cell_beg -1, or cell_beg and cell_end alike. */
 int lq_particle_interaction(const void* par_host, const void* par_device,
                             const float* pospres, const float* velrhop, const float* idep,
                             const float* str, const float* stn,

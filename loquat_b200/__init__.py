@@ -172,7 +172,7 @@ def grid_neighbor_search_noalloc(par_host, par_dev, pospres, part_cel, part_idx,
 # ------------------------------------------------------------------ operators
 def interaction_reserve(par_host) -> None:
     """lq_interaction_reserve: sizes particle_interaction's working arrays
-    for par_host's particle and cell counts, once, before a step loop."""
+    for par_host's particle counts, once, before a step loop."""
     check(lib().lq_interaction_reserve(ptr(par_host)), "lq_interaction_reserve")
 
 
