@@ -376,10 +376,9 @@ int scan_scratch_bytes(int ncell, size_t* bytes)
 /* --------------------------------------------- identities of the grids */
 namespace {
 
-/* `started`: ident holds the identity of each of np slots.  Not so before
- * a grid's first search, nor after a search over another particle count,
- * which does not follow the other slots' particles: the next search over np
- * particles then starts them again, on its own stream. */
+/* `started`: ident holds the identity of each of np slots.  Not so after a
+ * search over another particle count, which does not follow the other slots'
+ * particles: the next search over np particles then starts them again. */
 struct IdentityRecord {
     int* ident = nullptr;
     int* tmp = nullptr;
@@ -506,6 +505,30 @@ int bounds_count_grid(unsigned long long* v)
     return LQ_OK;
 }
 
+namespace {
+
+__global__ void __launch_bounds__(kBlock) k_iota(int n, int* __restrict__ p)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = i;
+}
+
+/* p[i] = i, there when the call returns, whatever stream reads it next. */
+int fill_identities(int n, int* p)
+{
+    if (n <= 0) return LQ_OK;
+    cudaStream_t s = nullptr;
+    LQ_TRY_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "grid identities");
+    k_iota<<<blocks_for(n), kBlock, 0, s>>>(n, p);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    LQ_TRY_CUDA(e, "grid identities");
+    return LQ_OK;
+}
+
+}  // namespace
+
 int identity_reset(const int* key, int np)
 {
     std::lock_guard<std::mutex> lock(g_id_mu);
@@ -526,7 +549,9 @@ int identity_reset(const int* key, int np)
         r.np = np;
     }
     r.gen = ++g_id_gen;
-    r.started = false;      /* the first search starts the identities */
+    r.started = false;
+    LQ_TRY(fill_identities(np, r.ident));
+    r.started = true;
     return LQ_OK;
 }
 

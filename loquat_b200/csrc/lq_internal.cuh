@@ -131,10 +131,10 @@ int grid_search(const Parameters* par_host, const Parameters* par_dev, const flo
 
 /* Particle identities of the drop-in grids (lq_grid_* and LoquatGrid),
  * keyed by the grid's cell_beg array: ident[slot] is the slot the particle
- * now there had before the search that started them, the first one over
- * the grid's full particle count, updated by every later search through the
- * grid's part_idx.  A search over another count ends them (the interaction
- * then builds its lists afresh) until the next full one.  A caller
+ * now there had when the grid was sized (its order before the first
+ * search), updated by every search through the grid's part_idx.  A search
+ * over another count ends them (the interaction then builds its lists
+ * afresh); the next full one starts them again.  A caller
  * that re-sorts its arrays after each search, as the reference does,
  * keeps its particles and these identities in step, which lets the
  * drop-in interaction carry neighbour lists across searches.  `gen`
